@@ -97,6 +97,41 @@ __host__ __device__ inline PackedEdge packEdge(const cn_soft_edge &e)
     return PackedEdge{e.particle_a, e.particle_b | (e.enabled ? 0u : 0x80000000u), e.rest_length, e.compliance};
 }
 
+// Tiled soft iteration (cn_tiles.h): one CTA per tile runs a stage -- the edges, then the tets or the
+// bends and dihedrals with the particle-rigid contacts -- on the particles the tile owns.
+struct TileHead {
+    uint32_t own, ownCount, halo, haloCount;   // ranges of TileSet::own / halo
+    uint32_t entry[2], entryCount[2];          // per stage: its entries
+    uint32_t slots[2];                         // per stage: record slots in shared memory
+    uint32_t bends, reserved;                  // stage 1 holds bends and dihedrals (else tets)
+};
+constexpr uint32_t kTileMaxRecords = 1023u;
+constexpr uint32_t kTileNoSlot = 0xffffu;
+// An own particle's records in a stage: first slot, distance between two, count.
+__host__ __device__ inline uint32_t tileRecord(uint32_t base, uint32_t width, uint32_t count)
+{
+    return base | ((width & 31u) << 16) | (count << 21);
+}
+__host__ __device__ inline uint32_t tileRecordBase(uint32_t r) { return r & 0xffffu; }
+__host__ __device__ inline uint32_t tileRecordWidth(uint32_t r) { return ((r >> 16) & 31u) ? ((r >> 16) & 31u) : 32u; }
+__host__ __device__ inline uint32_t tileRecordCount(uint32_t r) { return r >> 21; }
+
+struct TileSet {
+    uint32_t tiles = 0, tetTiles = 0;          // the tiles of tets come first
+    uint32_t entries[2] = {0, 0};
+    uint32_t smem[2] = {0, 0};
+    const TileHead *heads = nullptr;
+    const uint32_t *own = nullptr, *halo = nullptr;
+    const uint32_t *rec[2] = {};               // per own particle (tileRecord)
+    const uint32_t *id[2] = {};                // per entry: constraint (bends first, then dihedrals)
+    const uint2 *edges = nullptr;              // local particles (16 bits each), then their record slots
+    const uint4 *elems = nullptr;              // the same for four particles
+    float2 *ra[2] = {};                        // rest value, compliance / dt^2 (< 0: disabled), once per frame
+    float *lambda[2] = {};
+    float4 *xB = nullptr;                      // positions between the two stages
+};
+constexpr uint32_t kResidentSmemCap = 220u << 10;
+
 struct Scene {
     // per-tick work lists of a batch (all null for a single world)
     WorkList wP, wE, wT, wB, wC;      // particles, edges, tets, rigid bodies, colliders
@@ -187,6 +222,8 @@ struct Scene {
     const float4 *colMat = nullptr;
     float4 *prevBodyPos = nullptr, *prevBodyRot = nullptr;
     float4 *predBodyPos = nullptr, *predBodyRot = nullptr, *predBodyLin = nullptr, *predBodyAng = nullptr;
+    // without dynamic bodies: the predict's normalised orientations, for the contacts
+    float4 *prevBodyUnit = nullptr, *predBodyUnit = nullptr;
     float4 *colAabbMin = nullptr, *colAabbMax = nullptr;
     // rigid-rigid contacts (scenes with dynamic bodies): LBVH over the query-order colliders, the
     // moving colliders' candidate pairs, one contact per pair, body-pair groups for the velocities
@@ -381,6 +418,12 @@ void launchApplyBodyTargets(const Scene &s, const BodyTarget *list, const uint32
 void launchRigidPredict(const Scene &s, float dt, float gx, float gy, float gz, cudaStream_t st);
 // The LBVH over the query-order colliders' world AABBs (cn_rigid.cu), after the rigid predict.
 void launchColliderBvh(const Scene &s, void *scratch, cudaStream_t st);
+// The rigid predict and launchPredictAndKeys in one launch (a single world of few bodies without proxy
+// particles); false when the scene takes the two.
+bool launchPredictWorld(const Scene &s, float dt, const Config &c, cudaStream_t st);
+// launchUpdateVelocities, launchRigidContactVelocities and launchCopyPredictedRigid in one launch (a
+// single world without dynamic bodies, fluid and particle-particle contacts).
+void launchFinishSubstep(const Scene &s, float dt, uint32_t contactIterations, const Config &c, cudaStream_t st);
 void launchPredictAndKeys(const Scene &s, float dt, const Config &c, cudaStream_t st);
 void launchCellSetup(const Scene &s, uint32_t *scanTmp, void *sortScratch, cudaStream_t st);
 // Neighbour and superset lists: entry k of compute slot i at k * N + i (true) or i * cap + k.
@@ -403,9 +446,11 @@ void launchFluidVorticity(const Scene &s, float dt, cudaStream_t st);
 // particle-rigid contacts follow the soft families directly: no particle-particle contacts) and
 // a tet family, those contacts run in the tet gather's pass; returns true when they did, and the
 // caller launches them itself otherwise.
-bool launchSoftIteration(const Scene &s, float dt, const Config &c, cudaStream_t st, bool rigidContacts = false);
+// `first`: the substep's first iteration (a single world's edge and tet lambdas start at zero there; a
+// batch clears them).
+bool launchSoftIteration(const Scene &s, float dt, const Config &c, cudaStream_t st, bool first, bool rigidContacts = false);
 // The same for the families whose bit (1 << kFam*) is set in `families`, in the family order.
-bool launchSoftFamilies(const Scene &s, float dt, const Config &c, cudaStream_t st, uint32_t families,
+bool launchSoftFamilies(const Scene &s, float dt, const Config &c, cudaStream_t st, uint32_t families, bool first,
                         bool rigidContacts = false);
 constexpr uint32_t kAllFamilies = (1u << kFamilies) - 1u;
 // The XPBD schedule of a solver: CN_XPBD_* and, for the coloured schedules, each family's colour
@@ -418,7 +463,7 @@ struct XpbdPlan {
     const uint32_t *devStarts[kFamilies] = {};
 };
 bool launchSoftIteration(const Scene &s, float dt, const Config &c, const XpbdPlan &plan, cudaStream_t st,
-                         bool rigidContacts = false);
+                         bool first, bool rigidContacts = false);
 // Fused iterations: one thread-block cluster runs every iteration of a substep (soft families in
 // `plan`'s schedule, then the particle-rigid contacts when `rigid`), phases separated by cluster
 // barriers.  fusedIterationsShape() is {0, 0} when the cluster launch is unavailable.
@@ -449,6 +494,21 @@ void launchBatchFusedIterations(const Scene &s, const Config &c, float dt, const
 // scene's sums to x over the family's particle window.
 void launchBatchColourIteration(const Scene &s, float dt, const Config &c, uint32_t schedule, const uint32_t maxColours[2],
                                 const uint2 *scenes, const uint32_t *sceneCount, uint32_t grid, cudaStream_t st);
+// Tiled soft iterations: the entries' rest values and scaled compliances, read from the constraint
+// records at the start of every frame, then per iteration the two stages.  `flags`: the substep's first
+// soft iteration (lambdas start at zero) and its last; `contacts`: the iteration's particle-rigid
+// contacts run in the second stage.
+enum : uint32_t { kTileFirst = 1u, kTileLast = 2u };
+void launchTilePrepare(const Scene &s, const TileSet &t, float dt, cudaStream_t st);
+void launchTileEdges(const Scene &s, const TileSet &t, const Config &c, uint32_t flags, cudaStream_t st);
+void launchTileTets(const Scene &s, const TileSet &t, const Config &c, uint32_t flags, bool contacts, cudaStream_t st);
+void launchTileBends(const Scene &s, const TileSet &t, const Config &c, uint32_t flags, bool contacts, cudaStream_t st);
+// Every iteration of a substep of a coloured schedule in one CTA, the positions in its shared memory.
+bool residentColourFits(const Scene &s, const XpbdPlan &plan);
+void launchResidentColour(const Scene &s, const Config &c, float dt, const XpbdPlan &plan, uint32_t iterations,
+                          uint32_t softIterations, uint32_t contactIterations, bool rigid, cudaStream_t st);
+// Allows the kernels `bytes` of dynamic shared memory per CTA; false when the device has less.
+bool tileKernelsFit(uint32_t bytes);
 void launchFusedIterations(const Scene &s, const Config &c, float dt, const XpbdPlan &plan, uint32_t iterations,
                            uint32_t softIterations, uint32_t contactIterations, bool rigid, const FusedShape &shape,
                            cudaStream_t st);

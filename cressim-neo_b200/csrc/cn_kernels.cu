@@ -16,6 +16,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstdlib>
+#include <type_traits>
 #include <utility>
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -77,7 +78,7 @@ inline unsigned softBlocksFor(size_t n) { return n == 0 ? 1u : unsigned((n + kSo
 inline unsigned softGridFor(const WorkList &w, size_t n) { return w.tiles ? w.grid : softBlocksFor(n); }
 inline unsigned softApplyGrid(const Scene &s, uint2 win)
 {
-    return s.wP.tiles ? gridFor(s.wP, s.N) : softBlocksFor(win.y > win.x ? win.y - win.x : 0u);
+    return s.wP.tiles ? gridFor(s.wP, s.N) : softBlocksFor(win.y > win.x ? size_t(win.y - win.x) * 4u : 0u);
 }
 
 // Launches `k` with programmatic stream serialization (the kernel starts with pdlEnter()), so its
@@ -156,6 +157,10 @@ __device__ __forceinline__ void rigidPredictBody(const Scene &s, float dt, float
         s.predBodyRot[b] = integrateOrientation(q, xyz(ang), dt);
         s.predBodyLin[b] = mk4(l, lin.w);
         s.predBodyAng[b] = ang;
+    }
+    if (!s.hasDynamic) { // what the contacts normalise for every pair of every iteration
+        s.prevBodyUnit[b] = qNormalize(q);
+        s.predBodyUnit[b] = qNormalize(s.predBodyRot[b]);
     }
 }
 
@@ -323,6 +328,23 @@ __device__ __forceinline__ void predictParticle(const Scene &s, float dt, float 
     const uint32_t key = cellKey(cx, cy, cz);
     s.entries[i] = make_int4(cx, cy, cz, int(key));
     s.keysA[i] = key;
+}
+
+// The rigid predict (one block for a few bodies and colliders) and the particles', which do not read one
+// another: the last block takes the bodies.  Not for rigid proxy particles, placed at the predicted poses.
+__global__ void __launch_bounds__(kThreads) k_predictWorld(Scene s, float dt, float gx, float gy, float gz, bool writeKeys)
+{
+    if (blockIdx.x + 1u == gridDim.x) {
+        for (uint32_t b = threadIdx.x; b < s.B; b += blockDim.x) rigidPredictBody(s, dt, gx, gy, gz, b);
+        __syncthreads();
+        for (uint32_t c = threadIdx.x; c < s.C; c += blockDim.x) {
+            colliderAabb(s, c);
+            colliderFrame(s, c);
+        }
+        return;
+    }
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < s.N) predictParticle(s, dt, gx, gy, gz, writeKeys, i);
 }
 
 __global__ void __launch_bounds__(kThreads) k_predictKeys(Scene s, float dt, float gx, float gy, float gz,
@@ -699,6 +721,46 @@ __global__ void __launch_bounds__(kThreads) k_rigidCandidates(Scene s, const uin
             rigidCandidatesAt<1u>(s, i, s.candOffset[i]);
         }
     });
+}
+
+// The same for a few particles in one block: counts, their exclusive scan and the pairs, chunk by chunk
+// with a running carry (the offsets of the three launches it stands for).
+constexpr uint32_t kCandidateBlock = 512u;
+constexpr uint32_t kCandidateSmall = 2u * kCandidateBlock; // more chunks in turn cost more than the two launches saved
+__global__ void __launch_bounds__(kCandidateBlock) k_rigidCandidatesSmall(Scene s)
+{
+    __shared__ uint32_t warpSums[kCandidateBlock / 32u];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint32_t carry = 0;
+    for (uint32_t base = 0; base < s.N; base += kCandidateBlock) {
+        const uint32_t i = base + threadIdx.x;
+        const uint32_t count = i < s.N ? rigidCandidatesAt<0u>(s, i, 0u) : 0u;
+        uint32_t x = count;
+#pragma unroll
+        for (uint32_t o = 1; o < 32u; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31u) warpSums[warp] = x;
+        __syncthreads();
+        uint32_t before = 0, total = 0;
+        for (uint32_t w = 0; w < kCandidateBlock / 32u; ++w) {
+            if (w < warp) before += warpSums[w];
+            total += warpSums[w];
+        }
+        const uint32_t offset = carry + before + x - count;
+        if (i < s.N) {
+            s.candCount[i] = count;
+            s.candOffset[i] = offset;
+            if (count) rigidCandidatesAt<1u>(s, i, offset);
+        }
+        carry += total;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0u) {
+        s.meta_->requiredRigidPairs = carry;
+        s.meta_->rigidPairCount = min(carry, s.rigidPairCapacity);
+    }
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1361,15 +1423,19 @@ __device__ __forceinline__ float4 recordAt(const float4 *corr, uint32_t slot)
     return slot != kNoSlot ? corr[slot] : make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
-// physics_soft_solve_edge_constraints.cs.hlsl:10-74: one edge's corrections (zero when it is
-// disabled or degenerate) and, when it returns true, its new lambda.
-__device__ __forceinline__ bool edgeSolve(const Scene &s, float dt, float relax, const PackedEdge &ed, float lambda,
-                                          float &newLambda, float4 &cA, float4 &cB)
+// XPBD compliance over dt^2, as every family's shader takes it.
+__device__ __forceinline__ float scaledCompliance(float compliance, float dt)
 {
-    cA = make_float4(0.f, 0.f, 0.f, 0.f);
+    return mx(compliance, 0.0f) / mx(dt * dt, kEps);
+}
+
+// physics_soft_solve_edge_constraints.cs.hlsl:10-74: one edge's corrections (zero when it is
+// degenerate) and, when it returns true, its new lambda.
+__device__ __forceinline__ bool edgeCorrect(const float4 a, const float4 b, float rest, float alpha, float relax,
+                                            float lambda, float &newLambda, f3 &cA, f3 &cB)
+{
+    cA = f3{0.f, 0.f, 0.f};
     cB = cA;
-    if (ed.b >> 31) return false; // disabled
-    const float4 a = s.x[ed.a], b = s.x[ed.b];
     const float wA = a.w, wB = b.w, wSum = wA + wB;
     const f3 delta = xyz(b) - xyz(a);
     const float l2 = dot(delta, delta);
@@ -1377,15 +1443,29 @@ __device__ __forceinline__ bool edgeSolve(const Scene &s, float dt, float relax,
     const float len = sqrtf(l2);
     const f3 gA = -delta / len;
     const f3 gB = -gA;
-    const float alpha = mx(ed.compliance, 0.0f) / mx(dt * dt, kEps);
-    const float Cv = len - ed.rest;
+    const float Cv = len - rest;
     const float den = wSum + alpha;
     if (!(den > kEps)) return false;
     const float dl = -(Cv + alpha * lambda) / den;
     newLambda = lambda + dl;
-    cA = mk4(wA * dl * gA * relax, 0.0f);
-    cB = mk4(wB * dl * gB * relax, 0.0f);
+    cA = wA * dl * gA * relax;
+    cB = wB * dl * gB * relax;
     return true;
+}
+
+// One edge from its record (zero corrections when it is disabled).
+__device__ __forceinline__ bool edgeSolve(const Scene &s, float dt, float relax, const PackedEdge &ed, float lambda,
+                                          float &newLambda, float4 &cA, float4 &cB)
+{
+    cA = make_float4(0.f, 0.f, 0.f, 0.f);
+    cB = cA;
+    if (ed.b >> 31) return false; // disabled
+    f3 a, b;
+    const bool solved = edgeCorrect(s.x[ed.a], s.x[ed.b], ed.rest, scaledCompliance(ed.compliance, dt), relax, lambda,
+                                    newLambda, a, b);
+    cA = mk4(a, 0.0f);
+    cB = mk4(b, 0.0f);
+    return solved;
 }
 
 __device__ __forceinline__ void solveEdge(const Scene &s, float dt, float relax, uint32_t e)
@@ -1400,10 +1480,33 @@ __device__ __forceinline__ void solveEdge(const Scene &s, float dt, float relax,
     putRecord(s.edgeCorr, d.y, cB);
 }
 
-__global__ void __launch_bounds__(kThreads) k_solveEdges(Scene s, float dt, float relax)
+__global__ void __launch_bounds__(kThreads) k_solveEdges(Scene s, float dt, float relax, bool first)
 {
+    if (s.wE.tiles) {
+        pdlEnter();
+        forEachElem(s.wE, s.E, [&](uint32_t e) { solveEdge(s, dt, relax, e); });
+        return;
+    }
+    // A single world: the record, its gather slots and lambda (last written by this family's solve an
+    // iteration ago, which the kernel this one follows has waited for) load ahead of the wait, so
+    // that one round trip for the two positions is what follows it.
+    const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
+    PackedEdge ed{};
+    float lambda = 0.0f;
+    uint2 d = make_uint2(kNoSlot, kNoSlot);
+    if (e < s.E) {
+        ed = s.edgesP ? s.edgesP[e] : packEdge(s.edges[e]);
+        lambda = first ? 0.0f : s.edgeLambda[e];
+        d = reinterpret_cast<const uint2 *>(s.edgeDst)[e];
+    }
     pdlEnter();
-    forEachElem(s.wE, s.E, [&](uint32_t e) { solveEdge(s, dt, relax, e); });
+    if (e >= s.E) return;
+    float newLambda;
+    float4 cA, cB;
+    const bool solved = edgeSolve(s, dt, relax, ed, lambda, newLambda, cA, cB);
+    if (solved || first) s.edgeLambda[e] = solved ? newLambda : lambda;
+    putRecord(s.edgeCorr, d.x, cA);
+    putRecord(s.edgeCorr, d.y, cB);
 }
 
 // Gather of the correction records: each particle's records sit contiguously at its incidence
@@ -1436,48 +1539,101 @@ __device__ __forceinline__ void applyGatherAt(const Scene &s, const uint2 *range
     if (p.w > kEps) s.x[i] = gatheredPosition(ranges, corr, i, p);
 }
 
+// A single world's gather: four lanes per particle, lane c summing component c of its records in list
+// order (the components are independent sums, so the bits are those of one thread's), sixteen records in
+// flight.  The range and the position are read ahead of the wait -- a gather follows its family's
+// solve, which moves no particle and has itself waited for the kernel that last did -- so the records
+// are the one round trip after it.
+constexpr uint32_t kGatherLanes = 4u;
+constexpr uint32_t kGatherAhead = 16u;
+struct GatherLane {
+    bool live;
+    uint32_t comp, at, first, count;
+    float x, w;
+    __device__ __forceinline__ GatherLane(const Scene &s, const uint2 *ranges, uint32_t i, uint32_t end)
+    {
+        comp = threadIdx.x % kGatherLanes;
+        live = i < end;
+        at = 4u * i + comp;
+        first = count = 0u;
+        x = w = 0.0f;
+        if (!live) return;
+        x = reinterpret_cast<const float *>(s.x)[at];
+        w = s.x[i].w;
+        const uint2 r = ranges[i];
+        first = r.x;
+        count = r.y;
+    }
+    __device__ __forceinline__ float sum(const float4 *corr) const
+    {
+        const float *src = reinterpret_cast<const float *>(corr + first) + comp;
+        float total = 0.0f;
+        for (uint32_t k = 0; k < count; k += kGatherAhead) {
+            float c[kGatherAhead];
+#pragma unroll
+            for (uint32_t j = 0; j < kGatherAhead; ++j)
+                if (k + j < count) c[j] = src[4u * (k + j)];
+#pragma unroll
+            for (uint32_t j = 0; j < kGatherAhead; ++j)
+                if (k + j < count) total += c[j];
+        }
+        return total;
+    }
+};
+
 // physics_soft_apply_edge_corrections.cs.hlsl:9-35, physics_soft_apply_tet_corrections.cs.hlsl:9-50,
 // physics_soft_apply_bend_corrections.cs.hlsl:9-51, physics_strand_apply_distance_corrections.cs.hlsl:9-38.
 // A single world applies over `win`, the particles [lo, hi) that the family touches (bodies are
 // contiguous in the particle order; the others have no records and keep x); a batch over its tiles.
 __global__ void __launch_bounds__(kThreads) k_applyGather(Scene s, const uint2 *ranges, const float4 *corr, uint2 win)
 {
-    pdlEnter();
     if (s.wP.tiles) {
+        pdlEnter();
         forEachElem(s.wP, s.N, [&](uint32_t i) { applyGatherAt(s, ranges, corr, i); });
         return;
     }
-    const uint32_t i = win.x + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < win.y) applyGatherAt(s, ranges, corr, i);
+    const GatherLane g(s, ranges, win.x + (blockIdx.x * blockDim.x + threadIdx.x) / kGatherLanes, win.y);
+    pdlEnter();
+    if (g.live && g.w > kEps && g.comp < 3u) reinterpret_cast<float *>(s.x)[g.at] = g.x + g.sum(corr);
 }
 
 // physics_soft_solve_tet_constraints.cs.hlsl:15-87: one tet's four corrections and its new
 // lambda; false when the tet keeps its previous corrections (no weight, or a degenerate one).
-__device__ __forceinline__ bool tetSolve(const Scene &s, float dt, float relax, const cn_soft_tet &tet, float lambda,
-                                         float &newLambda, float4 c[4])
+__device__ __forceinline__ bool tetCorrect(const float4 q0, const float4 q1, const float4 q2, const float4 q3, float rest,
+                                           float alpha, float relax, float lambda, float &newLambda, f3 c[4])
 {
-    const float4 q0 = s.x[tet.particle_indices[0]], q1 = s.x[tet.particle_indices[1]];
-    const float4 q2 = s.x[tet.particle_indices[2]], q3 = s.x[tet.particle_indices[3]];
     const float w0 = q0.w, w1 = q1.w, w2 = q2.w, w3 = q3.w;
     if ((w0 + w1 + w2 + w3) <= kEps) return false;
     const f3 p0 = xyz(q0), p1 = xyz(q1), p2 = xyz(q2), p3 = xyz(q3);
     const float sv = dot(cross(p1 - p0, p2 - p0), p3 - p0) / 6.0f;
     const float vs = (sv >= 0.0f) ? 1.0f : -1.0f;
-    const float Cv = fabsf(sv) - mx(tet.rest_volume, 0.0f);
+    const float Cv = fabsf(sv) - mx(rest, 0.0f);
     const f3 g0 = cross(p3 - p1, p2 - p1) * (vs / 6.0f);
     const f3 g1 = cross(p2 - p0, p3 - p0) * (vs / 6.0f);
     const f3 g2 = cross(p3 - p0, p1 - p0) * (vs / 6.0f);
     const f3 g3 = cross(p1 - p0, p2 - p0) * (vs / 6.0f);
     const float sg = w0 * dot(g0, g0) + w1 * dot(g1, g1) + w2 * dot(g2, g2) + w3 * dot(g3, g3);
-    const float alpha = mx(tet.compliance, 0.0f) / mx(dt * dt, kEps);
     const float den = sg + alpha;
     if (den <= kEps) return false;
     const float dl = -(Cv + alpha * lambda) / den;
     newLambda = lambda + dl;
-    c[0] = mk4(w0 * dl * g0 * relax, 0.0f);
-    c[1] = mk4(w1 * dl * g1 * relax, 0.0f);
-    c[2] = mk4(w2 * dl * g2 * relax, 0.0f);
-    c[3] = mk4(w3 * dl * g3 * relax, 0.0f);
+    c[0] = w0 * dl * g0 * relax;
+    c[1] = w1 * dl * g1 * relax;
+    c[2] = w2 * dl * g2 * relax;
+    c[3] = w3 * dl * g3 * relax;
+    return true;
+}
+
+__device__ __forceinline__ bool tetSolve(const Scene &s, float dt, float relax, const cn_soft_tet &tet, float lambda,
+                                         float &newLambda, float4 c[4])
+{
+    f3 v[4];
+    if (!tetCorrect(s.x[tet.particle_indices[0]], s.x[tet.particle_indices[1]], s.x[tet.particle_indices[2]],
+                    s.x[tet.particle_indices[3]], tet.rest_volume, scaledCompliance(tet.compliance, dt), relax, lambda,
+                    newLambda, v))
+        return false;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) c[k] = mk4(v[k], 0.0f);
     return true;
 }
 
@@ -1496,49 +1652,79 @@ __device__ __forceinline__ void solveTet(const Scene &s, float dt, float relax, 
     putRecord(s.tetCorr, d.w, c[3]);
 }
 
-__global__ void __launch_bounds__(kThreads) k_solveTets(Scene s, float dt, float relax)
+__global__ void __launch_bounds__(kThreads) k_solveTets(Scene s, float dt, float relax, bool first)
 {
+    if (s.wT.tiles) {
+        pdlEnter();
+        forEachElem(s.wT, s.T, [&](uint32_t t) { solveTet(s, dt, relax, t); });
+        return;
+    }
+    // as k_solveEdges: everything but the positions ahead of the wait
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    cn_soft_tet tet{};
+    float lambda = 0.0f;
+    uint4 d = make_uint4(kNoSlot, kNoSlot, kNoSlot, kNoSlot);
+    if (t < s.T) {
+        tet = s.tets[t];
+        lambda = first ? 0.0f : s.tetLambda[t];
+        d = reinterpret_cast<const uint4 *>(s.tetDst)[t];
+    }
     pdlEnter();
-    forEachElem(s.wT, s.T, [&](uint32_t t) { solveTet(s, dt, relax, t); });
+    if (t >= s.T) return;
+    float newLambda;
+    float4 c[4];
+    const bool solved = tetSolve(s, dt, relax, tet, lambda, newLambda, c);
+    if (solved || first) s.tetLambda[t] = solved ? newLambda : lambda;
+    if (!solved) return; // keeps the previous records
+    putRecord(s.tetCorr, d.x, c[0]);
+    putRecord(s.tetCorr, d.y, c[1]);
+    putRecord(s.tetCorr, d.z, c[2]);
+    putRecord(s.tetCorr, d.w, c[3]);
 }
 
-// physics_soft_solve_bend_constraints.cs.hlsl:20-86
-__device__ __forceinline__ void solveBendAt(const Scene &s, float dt, float relax, uint32_t b)
+// physics_soft_solve_bend_constraints.cs.hlsl:20-86: one 3-point bend's corrections (zero when it is
+// degenerate) and, when it returns true, its new lambda.
+__device__ __forceinline__ bool bendCorrect(const float4 q0, const float4 q1, const float4 q2, float rest, float alpha,
+                                            float relax, float lambda, float &newLambda, f3 c[3])
 {
-    const cn_soft_bend bd = s.bends[b];
-    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 o0 = z, o1 = z, o2 = z;
-    const float4 q0 = s.x[bd.particle0], q1 = s.x[bd.particle1], q2 = s.x[bd.particle2];
+    c[0] = c[1] = c[2] = f3{0.f, 0.f, 0.f};
     const float w0 = q0.w, w1 = q1.w, w2 = q2.w;
     const f3 e0 = xyz(q0) - xyz(q1), e1 = xyz(q2) - xyz(q1);
     const float l0s = dot(e0, e0), l1s = dot(e1, e1);
-    if (w0 + w1 + w2 > kEps && l0s > kEps && l1s > kEps) {
-        const float l0 = sqrtf(l0s), l1 = sqrtf(l1s);
-        const f3 d0 = e0 / l0, d1 = e1 / l1;
-        const float ct = mn(mx(dot(d0, d1), -1.0f + 1.0e-4f), 1.0f - 1.0e-4f);
-        const float st2 = mx(1.0f - ct * ct, 1.0e-8f);
-        const float st = sqrtf(st2);
-        const float theta = acosf(ct);
-        const f3 g0 = -(d1 - ct * d0) / mx(l0 * st, kEps);
-        const f3 g2 = -(d0 - ct * d1) / mx(l1 * st, kEps);
-        const f3 g1 = -(g0 + g2);
-        const float den = w0 * dot(g0, g0) + w1 * dot(g1, g1) + w2 * dot(g2, g2);
-        const float alpha = mx(bd.compliance, 0.0f) / mx(dt * dt, kEps);
-        if (den + alpha > kEps) {
-            const float Cv = theta - bd.rest_angle;
-            const float lambda = s.bendLambda[b];
-            const float dl = -(Cv + alpha * lambda) / (den + alpha);
-            s.bendLambda[b] = lambda + dl;
-            o0 = mk4(w0 * dl * g0 * relax, 0.0f);
-            o1 = mk4(w1 * dl * g1 * relax, 0.0f);
-            o2 = mk4(w2 * dl * g2 * relax, 0.0f);
-        }
-    }
+    if (!(w0 + w1 + w2 > kEps && l0s > kEps && l1s > kEps)) return false;
+    const float l0 = sqrtf(l0s), l1 = sqrtf(l1s);
+    const f3 d0 = e0 / l0, d1 = e1 / l1;
+    const float ct = mn(mx(dot(d0, d1), -1.0f + 1.0e-4f), 1.0f - 1.0e-4f);
+    const float st2 = mx(1.0f - ct * ct, 1.0e-8f);
+    const float st = sqrtf(st2);
+    const float theta = acosf(ct);
+    const f3 g0 = -(d1 - ct * d0) / mx(l0 * st, kEps);
+    const f3 g2 = -(d0 - ct * d1) / mx(l1 * st, kEps);
+    const f3 g1 = -(g0 + g2);
+    const float den = w0 * dot(g0, g0) + w1 * dot(g1, g1) + w2 * dot(g2, g2);
+    if (!(den + alpha > kEps)) return false;
+    const float Cv = theta - rest;
+    const float dl = -(Cv + alpha * lambda) / (den + alpha);
+    newLambda = lambda + dl;
+    c[0] = w0 * dl * g0 * relax;
+    c[1] = w1 * dl * g1 * relax;
+    c[2] = w2 * dl * g2 * relax;
+    return true;
+}
+
+__device__ __forceinline__ void solveBendAt(const Scene &s, float dt, float relax, uint32_t b)
+{
+    const cn_soft_bend bd = s.bends[b];
+    float newLambda;
+    f3 c[3];
+    if (bendCorrect(s.x[bd.particle0], s.x[bd.particle1], s.x[bd.particle2], bd.rest_angle,
+                    scaledCompliance(bd.compliance, dt), relax, s.bendLambda[b], newLambda, c))
+        s.bendLambda[b] = newLambda;
     const uint4 d = reinterpret_cast<const uint4 *>(s.bendDst)[b];
-    putRecord(s.bendCorr, d.x, o0);
-    putRecord(s.bendCorr, d.y, o1);
-    putRecord(s.bendCorr, d.z, o2);
-    putRecord(s.bendCorr, d.w, z);
+    putRecord(s.bendCorr, d.x, mk4(c[0], 0.0f));
+    putRecord(s.bendCorr, d.y, mk4(c[1], 0.0f));
+    putRecord(s.bendCorr, d.z, mk4(c[2], 0.0f));
+    putRecord(s.bendCorr, d.w, make_float4(0.f, 0.f, 0.f, 0.f));
 }
 
 __global__ void __launch_bounds__(kThreads) k_solveBends(Scene s, float dt, float relax)
@@ -1548,31 +1734,20 @@ __global__ void __launch_bounds__(kThreads) k_solveBends(Scene s, float dt, floa
     if (b < s.Bn) solveBendAt(s, dt, relax, b);
 }
 
-// physics_cloth_solve_dihedral_constraints.cs.hlsl:20-95
-__device__ __forceinline__ void solveDihedralAt(const Scene &s, float dt, float relax, uint32_t d)
+// physics_cloth_solve_dihedral_constraints.cs.hlsl:20-95: the corrections of the two edge particles,
+// then the two opposite ones (zero when it is degenerate), and, when it returns true, the new lambda.
+__device__ __forceinline__ bool dihedralCorrect(const float4 e0m, const float4 e1m, const float4 o0m, const float4 o1m,
+                                                float rest, float alpha, float relax, float lambda, float &newLambda,
+                                                f3 c[4])
 {
-    const uint32_t ci = s.Bn + d;
-    const cn_cloth_dihedral h = s.dihedrals[d];
-    const uint4 dst = reinterpret_cast<const uint4 *>(s.bendDst)[ci];
-    auto put4 = [&](float4 a, float4 b, float4 c, float4 e) {
-        putRecord(s.bendCorr, dst.x, a);
-        putRecord(s.bendCorr, dst.y, b);
-        putRecord(s.bendCorr, dst.z, c);
-        putRecord(s.bendCorr, dst.w, e);
-    };
-    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 e0m = s.x[h.edge_particle0], e1m = s.x[h.edge_particle1];
-    const float4 o0m = s.x[h.opposite_particle0], o1m = s.x[h.opposite_particle1];
+    c[0] = c[1] = c[2] = c[3] = f3{0.f, 0.f, 0.f};
     const f3 p0 = xyz(o0m), p1 = xyz(o1m), p2 = xyz(e0m), p3 = xyz(e1m);
     const f3 edge = p3 - p2;
     const float el2 = dot(edge, edge);
     const f3 rn0 = cross(p2 - p0, p3 - p0);
     const f3 rn1 = cross(p3 - p1, p2 - p1);
     const float n0s = dot(rn0, rn0), n1s = dot(rn1, rn1);
-    if (el2 <= kEps || n0s <= kEps || n1s <= kEps) {
-        put4(z, z, z, z);
-        return;
-    }
+    if (el2 <= kEps || n0s <= kEps || n1s <= kEps) return false;
     const float el = sqrtf(el2);
     const float iel = 1.0f / el;
     const f3 sn0 = rn0 / n0s, sn1 = rn1 / n1s;
@@ -1583,20 +1758,35 @@ __device__ __forceinline__ void solveDihedralAt(const Scene &s, float dt, float 
     const f3 n0 = rn0 / sqrtf(n0s), n1 = rn1 / sqrtf(n1s);
     const float theta = atan2f(dot(edge * iel, cross(n0, n1)), mn(mx(dot(n0, n1), -1.0f), 1.0f));
     const float twoPi = 6.283185307179586f;
-    float Cv = theta - h.rest_angle;
+    float Cv = theta - rest;
     Cv = Cv - twoPi * floorf((Cv + 3.141592653589793f) / twoPi);
     const float w0 = e0m.w, w1 = e1m.w, w2 = o0m.w, w3 = o1m.w;
     const float den = w0 * dot(g0, g0) + w1 * dot(g1, g1) + w2 * dot(g2, g2) + w3 * dot(g3, g3);
-    const float alpha = mx(h.compliance, 0.0f) / mx(dt * dt, kEps);
-    if (den + alpha <= kEps) {
-        put4(z, z, z, z);
-        return;
-    }
-    const float lambda = s.bendLambda[ci];
+    if (den + alpha <= kEps) return false;
     const float dl = -(Cv + alpha * lambda) / (den + alpha);
-    s.bendLambda[ci] = lambda + dl;
-    put4(mk4(w0 * dl * g0 * relax, 0.0f), mk4(w1 * dl * g1 * relax, 0.0f), mk4(w2 * dl * g2 * relax, 0.0f),
-         mk4(w3 * dl * g3 * relax, 0.0f));
+    newLambda = lambda + dl;
+    c[0] = w0 * dl * g0 * relax;
+    c[1] = w1 * dl * g1 * relax;
+    c[2] = w2 * dl * g2 * relax;
+    c[3] = w3 * dl * g3 * relax;
+    return true;
+}
+
+__device__ __forceinline__ void solveDihedralAt(const Scene &s, float dt, float relax, uint32_t d)
+{
+    const uint32_t ci = s.Bn + d;
+    const cn_cloth_dihedral h = s.dihedrals[d];
+    const uint4 dst = reinterpret_cast<const uint4 *>(s.bendDst)[ci];
+    float newLambda;
+    f3 c[4];
+    if (dihedralCorrect(s.x[h.edge_particle0], s.x[h.edge_particle1], s.x[h.opposite_particle0],
+                        s.x[h.opposite_particle1], h.rest_angle, scaledCompliance(h.compliance, dt), relax,
+                        s.bendLambda[ci], newLambda, c))
+        s.bendLambda[ci] = newLambda;
+    putRecord(s.bendCorr, dst.x, mk4(c[0], 0.0f));
+    putRecord(s.bendCorr, dst.y, mk4(c[1], 0.0f));
+    putRecord(s.bendCorr, dst.z, mk4(c[2], 0.0f));
+    putRecord(s.bendCorr, dst.w, mk4(c[3], 0.0f));
 }
 
 __global__ void __launch_bounds__(kThreads) k_solveDihedrals(Scene s, float dt, float relax)
@@ -2005,8 +2195,71 @@ __device__ __forceinline__ ContactParticle loadContactParticle(const Scene &s, u
     return p;
 }
 
+// The world frame of a collider as the contacts use it: centre, orientation and shape extents.  Without
+// dynamic bodies the poses are those of the substep's predict, whose colliderFrame holds the same values
+// (the same expressions); bodies that move between the iterations have it evaluated from their pose.
+struct ContactFrame {
+    f3 centre;
+    float4 rotation;
+    float4 e0, e1;
+};
+
+__device__ __forceinline__ ContactFrame contactFrame(const Scene &s, uint32_t c, const cn_collider_broadphase &bp, uint32_t b,
+                                                     const f3 bpos, const float4 rot)
+{
+    ContactFrame f;
+    if (!s.hasDynamic && bp.owner_body == b) {
+        const float4 *fr = s.colFrame + size_t(c) * 4;
+        const float4 f0 = fr[0];
+        f.rotation = fr[1];
+        f.e0 = fr[2];
+        f.e1 = fr[3];
+        f.centre = xyz(f0);
+        return f;
+    }
+    const float4 bq = qNormalize(rot), bsc = s.bodyScale[b];
+    const cn_collider_geometry cg = s.colGeo[c];
+    const f3 clp{cg.local_position[0], cg.local_position[1], cg.local_position[2]};
+    const float4 clq = qNormalize(make_float4(cg.local_orientation[0], cg.local_orientation[1], cg.local_orientation[2],
+                                              cg.local_orientation[3]));
+    f.centre = bpos + qRotate(bq, clp);
+    f.rotation = qNormalize(qMul(bq, clq));
+    const float4 sp4 = make_float4(cg.shape_params[0], cg.shape_params[1], cg.shape_params[2], cg.shape_params[3]);
+    f.e0 = f.e1 = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (bp.shape_type == CN_COLLIDER_SPHERE) {
+        f.e0.x = sphereRadius(sp4, bsc);
+    } else if (bp.shape_type == CN_COLLIDER_BOX) {
+        f.e0 = mk4(boxHalfExtents(sp4, bsc), 0.f);
+    } else {
+        f3 a, b2;
+        float cap = 0.0f;
+        capsuleSegment(f.centre, f.rotation, sp4, bsc, a, b2, cap);
+        f.e0 = mk4(a, cap);
+        f.e1 = mk4(b2, 0.f);
+    }
+    return f;
+}
+
+// The candidates of a particle and, looked up with them, the first pair's body and its first collider:
+// the dependent loads of a contact that do not need the particle's position.
+struct ContactRange {
+    uint32_t count, first, body, collider, colliders;
+};
+
+__device__ __forceinline__ ContactRange contactRange(const Scene &s, uint32_t i)
+{
+    ContactRange r{s.candCount[i], s.candOffset[i], 0u, 0u, 0u};
+    if (r.count == 0u) return r;
+    r.body = s.rigidPairs[min(r.first, s.rigidPairCapacity - 1u)].y; // past a full buffer: not used
+    if (r.body >= s.B) return r;
+    const uint2 cr = s.bodyColRanges[r.body];
+    r.colliders = cr.y;
+    if (cr.y) r.collider = s.bodyColIdx[cr.x];
+    return r;
+}
+
 __device__ __forceinline__ RigidContact generateRigidContact(const Scene &s, uint32_t i, uint32_t b,
-                                                             const ContactParticle &pt)
+                                                             const ContactParticle &pt, uint32_t colliders, uint32_t collider0)
 {
     RigidContact out{};
     if (pt.proxy) return out;
@@ -2014,57 +2267,58 @@ __device__ __forceinline__ RigidContact generateRigidContact(const Scene &s, uin
     const float sr = pt.radius;
     const uint4 m = pt.meta;
     const f3 bpos = xyz(s.predBodyPos[b]);
-    const float4 bq = qNormalize(s.predBodyRot[b]);
-    const float4 bsc = s.bodyScale[b];
-    const uint2 cr = s.bodyColRanges[b];
+    const float4 rot = s.predBodyRot[b];
     float bestPen = 0.0f;
     uint32_t bestCol = 0;
     f3 bestN{0.f, 1.f, 0.f}, bestW{0.f, 0.f, 0.f};
     for (uint32_t k = 0; k < kColliderIterationCap; ++k) {
-        if (k >= cr.y) break;
-        const uint32_t c = s.bodyColIdx[cr.x + k];
+        if (k >= colliders) break;
+        const uint32_t c = k == 0u ? collider0 : s.bodyColIdx[s.bodyColRanges[b].x + k];
         const cn_collider_broadphase bp = s.colBp[c];
-        const cn_collider_geometry cg = s.colGeo[c]; // before the filter: same round trip as bp
+        const ContactFrame f = contactFrame(s, c, bp, b, bpos, rot); // before the filter: same round trip as bp
         if (bp.enabled_flag == 0u || bp.environment_index != m.x) continue;
         if ((m.w & bp.collision_layer) == 0u || (bp.collision_mask & m.z) == 0u) continue;
-        const f3 clp{cg.local_position[0], cg.local_position[1], cg.local_position[2]};
-        const float4 clq = qNormalize(make_float4(cg.local_orientation[0], cg.local_orientation[1],
-                                                  cg.local_orientation[2], cg.local_orientation[3]));
-        const f3 cwp = bpos + qRotate(bq, clp);
-        const float4 cwq = qNormalize(qMul(bq, clq));
-        const f3 pl = qInvRotate(cwq, sp - cwp);
-        f3 nl{0.f, 1.f, 0.f}, cw{0.f, 0.f, 0.f};
-        float sd = 0.0f;
-        const float4 sp4 = make_float4(cg.shape_params[0], cg.shape_params[1], cg.shape_params[2], cg.shape_params[3]);
+        // the signed distance, and what the normal and the surface point come from: they are only
+        // evaluated for a collider that is penetrated deeper than the ones before it
         if (bp.shape_type == CN_COLLIDER_SPHERE) {
-            const float r = sphereRadius(sp4, bsc);
+            const f3 pl = qInvRotate(f.rotation, sp - f.centre);
+            const float r = f.e0.x;
             const float l = sqrtf(dot(pl, pl));
-            nl = l > kEps ? (pl / l) : f3{0.f, 1.f, 0.f};
-            sd = l - r;
-            cw = cwp + qRotate(cwq, nl * r);
+            const float pen = sr - (l - r);
+            if (pen <= 0.0f || pen <= bestPen) continue;
+            const f3 nl = l > kEps ? (pl / l) : f3{0.f, 1.f, 0.f};
+            bestPen = pen;
+            bestCol = c;
+            bestN = safeNormalize(qRotate(f.rotation, nl), f3{0.f, 1.f, 0.f});
+            bestW = f.centre + qRotate(f.rotation, nl * r);
         } else if (bp.shape_type == CN_COLLIDER_BOX) {
-            const f3 he = boxHalfExtents(sp4, bsc);
+            const f3 pl = qInvRotate(f.rotation, sp - f.centre);
+            const f3 he = xyz(f.e0);
             const f3 cl = clamp3(pl, -he, he);
             const f3 d = pl - cl;
             const float dl = sqrtf(dot(d, d));
-            if (dl > kEps) {
+            const f3 ds = he - fabs3(pl);
+            const bool outside = dl > kEps;
+            const float pen = sr - (outside ? dl : -mn(ds.x, mn(ds.y, ds.z)));
+            if (pen <= 0.0f || pen <= bestPen) continue;
+            f3 nl, cs;
+            if (outside) {
                 nl = d / dl;
-                sd = dl;
-                cw = cwp + qRotate(cwq, cl);
+                cs = cl;
             } else {
                 nl = closestFaceNormalLocal(pl, he);
-                const f3 ds = he - fabs3(pl);
-                sd = -mn(ds.x, mn(ds.y, ds.z));
-                f3 cs = pl;
+                cs = pl;
                 if (fabsf(nl.x) > 0.5f) cs.x = nl.x * he.x;
                 else if (fabsf(nl.y) > 0.5f) cs.y = nl.y * he.y;
                 else cs.z = nl.z * he.z;
-                cw = cwp + qRotate(cwq, cs);
             }
+            bestPen = pen;
+            bestCol = c;
+            bestN = safeNormalize(qRotate(f.rotation, nl), f3{0.f, 1.f, 0.f});
+            bestW = f.centre + qRotate(f.rotation, cs);
         } else {
-            f3 a, b2;
-            float cap = 0.0f;
-            capsuleSegment(cwp, cwq, sp4, bsc, a, b2, cap);
+            const f3 a = xyz(f.e0), b2 = xyz(f.e1);
+            const float cap = f.e0.w;
             const f3 seg = b2 - a;
             const float l2 = dot(seg, seg);
             float t = 0.0f;
@@ -2072,19 +2326,17 @@ __device__ __forceinline__ RigidContact generateRigidContact(const Scene &s, uin
             const f3 cl = lerp3(a, b2, t);
             const f3 d = sp - cl;
             const float l = sqrtf(dot(d, d));
+            const float pen = sr - (l - cap);
+            if (pen <= 0.0f || pen <= bestPen) continue;
             const f3 wn = l > kEps ? (d / l) : f3{1.f, 0.f, 0.f};
-            sd = l - cap;
-            nl = qInvRotate(cwq, wn);
-            cw = cl + wn * cap;
+            bestPen = pen;
+            bestCol = c;
+            bestN = safeNormalize(qRotate(f.rotation, qInvRotate(f.rotation, wn)), f3{0.f, 1.f, 0.f});
+            bestW = cl + wn * cap;
         }
-        const float pen = sr - sd;
-        if (pen <= 0.0f || pen <= bestPen) continue;
-        bestPen = pen;
-        bestCol = c;
-        bestN = safeNormalize(qRotate(cwq, nl), f3{0.f, 1.f, 0.f});
-        bestW = cw;
     }
     if (bestPen > 0.0f) {
+        const float4 bq = s.hasDynamic ? qNormalize(rot) : s.predBodyUnit[b];
         out.particle = i; out.body = b; out.collider = bestCol; out.active = 1u;
         out.normalPenetration = mk4(bestN, bestPen);
         out.rigidLocalPoint = mk4(qInvRotate(bq, bestW - bpos), 0.0f);
@@ -2099,24 +2351,42 @@ struct ContactCorrection {
     bool rigid;
 };
 
+// What the solve reads of the pair's body.
+struct ContactBody {
+    float4 prevPos, predPos, prevQ, predQ;
+    uint32_t type;
+};
+
+__device__ __forceinline__ ContactBody loadContactBody(const Scene &s, uint32_t b)
+{
+    ContactBody o;
+    o.prevPos = s.prevBodyPos[b];
+    o.predPos = s.predBodyPos[b];
+    o.prevQ = s.hasDynamic ? s.prevBodyRot[b] : s.prevBodyUnit[b];
+    o.predQ = s.hasDynamic ? s.predBodyRot[b] : s.predBodyUnit[b];
+    o.type = s.bodyType[b];
+    return o;
+}
+
 __device__ __forceinline__ ContactCorrection solveRigidContact(const Scene &s, const Config &cfg,
                                                                const RigidContact &c, float4 sp,
-                                                               const ContactParticle &pt)
+                                                               const ContactParticle &pt, const ContactBody &body)
 {
     ContactCorrection out{f3{0.f, 0.f, 0.f}, f3{0.f, 0.f, 0.f}, f3{0.f, 0.f, 0.f}, false};
     const uint32_t b = c.body;
     const float iS = sp.w;
     const f3 prevS = pt.prev;
-    const float4 prevB = s.prevBodyPos[b], predB = s.predBodyPos[b];
-    const float4 prevQ = qNormalize(s.prevBodyRot[b]), predQ = qNormalize(s.predBodyRot[b]);
-    const float iR = s.bodyType[b] == CN_BODY_DYNAMIC ? predB.w : 0.0f;
+    const float4 prevB = body.prevPos, predB = body.predPos;
+    const float4 prevQ = s.hasDynamic ? qNormalize(body.prevQ) : body.prevQ;
+    const float4 predQ = s.hasDynamic ? qNormalize(body.predQ) : body.predQ;
+    const float iR = body.type == CN_BODY_DYNAMIC ? predB.w : 0.0f;
     if (iS <= kEps && iR <= kEps) return out;
     const float pen = mn(mx(c.normalPenetration.w - cfg.slop, 0.0f), cfg.softMaxCorrection);
     if (pen <= 0.0f) return out;
     const f3 n = safeNormalize(xyz(c.normalPenetration), f3{0.f, 1.f, 0.f});
-    f3 inI = xyz(s.bodyInvInertia[b]);
+    const bool moves = iR > kEps; // only a body with weight takes a share
+    const f3 inI = moves ? xyz(s.bodyInvInertia[b]) : f3{0.f, 0.f, 0.f};
     const f3 mat = combineContactMaterial(pt.material, s.colMat[c.collider]);
-    if (iR <= kEps) inI = f3{0.f, 0.f, 0.f};
     const f3 prevCP = xyz(prevB) + qRotate(prevQ, xyz(c.rigidLocalPoint));
     const f3 cp = xyz(predB) + qRotate(predQ, xyz(c.rigidLocalPoint));
     const f3 rR = cp - xyz(predB);
@@ -2125,8 +2395,11 @@ __device__ __forceinline__ ContactCorrection solveRigidContact(const Scene &s, c
     if (denom <= kEps) return out;
     const float lambda = (pen / denom) * cfg.softContactRelaxation;
     f3 corr = n * (iS * lambda);
-    f3 rt = -n * (iR * lambda);
-    f3 rr = -mulWorldInvInertia(inI, predQ, cross(rR, n)) * lambda;
+    f3 rt{0.f, 0.f, 0.f}, rr{0.f, 0.f, 0.f};
+    if (moves) {
+        rt = -n * (iR * lambda);
+        rr = -mulWorldInvInertia(inI, predQ, cross(rR, n)) * lambda;
+    }
     const f3 relDisp = (cp - prevCP) - (xyz(sp) - prevS);
     const f3 fd = positionFrictionDelta(projectOntoTangent(relDisp, n), pen, mat.x, mat.z,
                                         cfg.positionFrictionMinDistance);
@@ -2138,8 +2411,10 @@ __device__ __forceinline__ ContactCorrection solveRigidContact(const Scene &s, c
         if (tden > kEps) {
             const float tl = fdist / tden;
             corr += t * (tl * iS * cfg.softContactRelaxation);
-            rt -= t * (tl * iR * cfg.softContactRelaxation);
-            rr -= mulWorldInvInertia(inI, predQ, cross(rR, t)) * (tl * cfg.softContactRelaxation);
+            if (moves) {
+                rt -= t * (tl * iR * cfg.softContactRelaxation);
+                rr -= mulWorldInvInertia(inI, predQ, cross(rR, t)) * (tl * cfg.softContactRelaxation);
+            }
         }
     }
     if (iS > kEps) out.soft = corr;
@@ -2151,31 +2426,37 @@ __device__ __forceinline__ ContactCorrection solveRigidContact(const Scene &s, c
     return out;
 }
 
-// Generate + solve every candidate pair of particle i (pairs are particle-major), then either
-// accumulate into posCorr (explicit contacts present) or apply directly
-// (physics_particle_apply_position_corrections.cs.hlsl:8-30).
-// Particle i's contacts from its position sp (its x, or the value the fused gather just computed).
-__device__ __forceinline__ void rigidContactsFrom(const Scene &s, const Config &cfg, bool applyDirect, uint32_t i,
-                                                  const float4 sp)
+// Generate + solve every candidate pair of particle i (pairs are particle-major) from its position sp
+// (its x, or the value the gather just computed): the summed correction; `any`: some contact added to
+// it.  `cnt` candidate pairs from `off`: the caller loads the range with the position (one round trip).
+// `store`: the pass writes its contact records.
+__device__ __forceinline__ f3 rigidContactsSum(const Scene &s, const Config &cfg, uint32_t i, const float4 sp,
+                                               const ContactRange &range, bool store, bool &any)
 {
-    const uint32_t cnt = s.candCount[i];
-    const uint32_t off = s.candOffset[i]; // with the count: one round trip fewer
     f3 corr{0.f, 0.f, 0.f};
-    bool any = false;
+    any = false;
     // A particle without weight takes no correction, and with no dynamic body nothing receives
     // its contacts' shares: only the stored records (the last contact iteration) need them.
-    const bool inert = sp.w <= kEps && !s.hasDynamic && !s.storeRigidContacts;
-    if (cnt && !inert) {
+    const bool inert = sp.w <= kEps && !s.hasDynamic && !store;
+    if (range.count && !inert) {
         const uint32_t lim = s.meta_->rigidPairCount;
         const ContactParticle pt = loadContactParticle(s, i, sp);
-        for (uint32_t k = 0; k < cnt; ++k) {
-            const uint32_t pi = off + k;
+        for (uint32_t k = 0; k < range.count; ++k) {
+            const uint32_t pi = range.first + k;
             if (pi >= lim) break;
-            const uint2 pr = s.rigidPairs[pi]; // pr.x == i: pairs are emitted particle-major
-            const RigidContact c = generateRigidContact(s, i, pr.y, pt);
-            if (s.storeRigidContacts) s.rigidContacts[pi] = c;
+            uint2 pr = make_uint2(i, range.body); // pairs are emitted particle-major
+            uint32_t colliders = range.colliders, collider0 = range.collider;
+            if (k) {
+                pr = s.rigidPairs[pi];
+                const uint2 cr = s.bodyColRanges[pr.y];
+                colliders = cr.y;
+                if (cr.y) collider0 = s.bodyColIdx[cr.x];
+            }
+            const ContactBody body = loadContactBody(s, pr.y); // with the collider's frame: one round trip
+            const RigidContact c = generateRigidContact(s, i, pr.y, pt, colliders, collider0);
+            if (store) s.rigidContacts[pi] = c;
             if (!c.active) continue;
-            const ContactCorrection d = solveRigidContact(s, cfg, c, sp, pt);
+            const ContactCorrection d = solveRigidContact(s, cfg, c, sp, pt, body);
             // the particle's float-atomic order of the reference == pair order here
             if (sp.w > kEps) {
                 corr = corr + d.soft;
@@ -2187,6 +2468,16 @@ __device__ __forceinline__ void rigidContactsFrom(const Scene &s, const Config &
             }
         }
     }
+    return corr;
+}
+
+// The contacts of particle i, accumulated into posCorr (explicit contacts present) or applied directly
+// (physics_particle_apply_position_corrections.cs.hlsl:8-30).
+__device__ __forceinline__ void rigidContactsFrom(const Scene &s, const Config &cfg, bool applyDirect, uint32_t i,
+                                                  const float4 sp, const ContactRange &range)
+{
+    bool any;
+    const f3 corr = rigidContactsSum(s, cfg, i, sp, range, s.storeRigidContacts != 0u, any);
     if (applyDirect) {
         // applyParticlePositionCorrections with an accumulator that only this pass wrote
         if (sp.w <= kEps) return;
@@ -2200,7 +2491,7 @@ __device__ __forceinline__ void rigidContactsFrom(const Scene &s, const Config &
 
 __device__ __forceinline__ void rigidContactsAt(const Scene &s, const Config &cfg, bool applyDirect, uint32_t i)
 {
-    rigidContactsFrom(s, cfg, applyDirect, i, s.x[i]);
+    rigidContactsFrom(s, cfg, applyDirect, i, s.x[i], contactRange(s, i));
 }
 
 __global__ void __launch_bounds__(kThreads) k_rigidContacts(Scene s, Config cfg, bool applyDirect)
@@ -2216,12 +2507,28 @@ __global__ void __launch_bounds__(kThreads) k_rigidContacts(Scene s, Config cfg,
 // particle) gives their results bit for bit with one launch and one pass over x fewer.
 __global__ void __launch_bounds__(kThreads) k_applyTetsRigidContacts(Scene s, Config cfg)
 {
+    if (!s.wP.tiles) { // a single world: the four-lane gather, its first lane runs the contacts
+        const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / kGatherLanes;
+        GatherLane g(s, s.tetRanges, i, s.N);
+        ContactRange range{};
+        if (g.live && g.comp == 0u) range = contactRange(s, i);
+        pdlEnter();
+        if (g.live && g.w > kEps && g.comp < 3u && i >= s.tetWin.x && i < s.tetWin.y) g.x += g.sum(s.tetCorr);
+        float4 p;
+        const uint32_t lane = threadIdx.x & 31u & ~(kGatherLanes - 1u);
+        p.x = __shfl_sync(0xffffffffu, g.x, lane);
+        p.y = __shfl_sync(0xffffffffu, g.x, lane + 1u);
+        p.z = __shfl_sync(0xffffffffu, g.x, lane + 2u);
+        p.w = g.w;
+        if (g.live && g.comp == 0u) rigidContactsFrom(s, cfg, true, i, p, range);
+        return;
+    }
     pdlEnter();
     // the gathered position goes to the contacts in registers: x is read and written once
     forEachElem(s.wP, s.N, [&](uint32_t i) {
         float4 p = s.x[i];
-        if (s.wP.tiles || (i >= s.tetWin.x && i < s.tetWin.y)) p = gatheredPosition(s.tetRanges, s.tetCorr, i, p);
-        rigidContactsFrom(s, cfg, true, i, p);
+        p = gatheredPosition(s.tetRanges, s.tetCorr, i, p);
+        rigidContactsFrom(s, cfg, true, i, p, contactRange(s, i));
     });
 }
 
@@ -2348,36 +2655,62 @@ __device__ __forceinline__ void rigidContactVelocitiesAt(const Scene &s, uint32_
     const float rpt = cfg.restitutionPenetrationThreshold;
     f3 vel = xyz(v0);
     const float vw = v0.w;
+    // What a contact's impulse needs beside the particle's velocity is the same in every iteration: the
+    // first kHeld contacts keep it in registers (ground and tool), later ones evaluate it each time.
+    struct Held {
+        bool active;
+        f3 n, rcv;
+        float nd, restitution;
+        bool bounces;
+    };
+    auto evaluate = [&](uint32_t pi) {
+        Held h{};
+        const RigidContact c = s.rigidContacts[pi];
+        h.active = c.active != 0u;
+        if (!h.active) return h;
+        const uint32_t b = c.body;
+        const float4 rp = s.predBodyPos[b];
+        const float iR = s.bodyType[b] == CN_BODY_DYNAMIC ? rp.w : 0.0f;
+        const float4 rq = qNormalize(s.predBodyRot[b]);
+        const f3 rl = xyz(s.predBodyLin[b]), ra = xyz(s.predBodyAng[b]);
+        const f3 inI = xyz(s.bodyInvInertia[b]);
+        h.n = safeNormalize(xyz(c.normalPenetration), f3{0.f, 1.f, 0.f});
+        const f3 cp = xyz(rp) + qRotate(rq, xyz(c.rigidLocalPoint));
+        const f3 rR = cp - xyz(rp);
+        h.rcv = rl + cross(ra, rR);
+        h.nd = iS + contactEffectiveMass(iR, inI, rq, rR, h.n);
+        h.restitution = saturate(combineContactMaterial(s.contactMaterials[s.matIdx[i]], s.colMat[c.collider]).y);
+        h.bounces = c.normalPenetration.w <= rpt;
+        return h;
+    };
+    constexpr uint32_t kHeld = 2u;
+    Held held[kHeld];
+#pragma unroll
+    for (uint32_t k = 0; k < kHeld; ++k) {
+        held[k].active = false;
+        if (k < cnt && off + k < lim) held[k] = evaluate(off + k);
+    }
     for (uint32_t it = 0; it < iterations; ++it) {
         f3 corr{0.f, 0.f, 0.f};
-        for (uint32_t k = 0; k < cnt; ++k) {
-            const uint32_t pi = off + k;
-            if (pi >= lim) break;
-            const RigidContact c = s.rigidContacts[pi];
-            if (!c.active) continue;
-            const uint32_t b = c.body;
-            const float4 rp = s.predBodyPos[b];
-            const float iR = s.bodyType[b] == CN_BODY_DYNAMIC ? rp.w : 0.0f;
-            const float4 rq = qNormalize(s.predBodyRot[b]);
-            const f3 rl = xyz(s.predBodyLin[b]), ra = xyz(s.predBodyAng[b]);
-            const f3 inI = xyz(s.bodyInvInertia[b]);
-            const f3 n = safeNormalize(xyz(c.normalPenetration), f3{0.f, 1.f, 0.f});
-            const f3 cp = xyz(rp) + qRotate(rq, xyz(c.rigidLocalPoint));
-            const f3 rR = cp - xyz(rp);
-            const f3 rcv = rl + cross(ra, rR);
-            const f3 rel = vel - rcv;
-            const float nv = dot(rel, n);
-            if (nv >= 0.0f) continue;
-            const float nd = iS + contactEffectiveMass(iR, inI, rq, rR, n);
-            if (nd <= kEps) continue;
-            const f3 mat = combineContactMaterial(s.contactMaterials[s.matIdx[i]], s.colMat[c.collider]);
-            const bool er = (-nv > cfg.restitutionVelocityThreshold) && (c.normalPenetration.w <= rpt);
-            const float rest = er ? saturate(mat.y) : 0.0f;
+        bool any = false;
+        auto impulse = [&](const Held &h) {
+            if (!h.active) return;
+            const f3 rel = vel - h.rcv;
+            const float nv = dot(rel, h.n);
+            if (nv >= 0.0f) return;
+            if (h.nd <= kEps) return;
+            const bool er = (-nv > cfg.restitutionVelocityThreshold) && h.bounces;
+            const float rest = er ? h.restitution : 0.0f;
             const float dnv = er ? (-rest * nv) : 0.0f;
-            const float imp = mx(0.0f, (dnv - nv) / nd);
-            corr = corr + (n * imp) * iS;
-        }
+            const float imp = mx(0.0f, (dnv - nv) / h.nd);
+            corr = corr + (h.n * imp) * iS;
+            any = true;
+        };
+#pragma unroll
+        for (uint32_t k = 0; k < kHeld; ++k) impulse(held[k]);
+        for (uint32_t k = kHeld; k < cnt && off + k < lim; ++k) impulse(evaluate(off + k));
         vel = vel + corr;
+        if (!any) break; // the velocity stays: so do the iterations that follow
     }
     s.v[i] = mk4(vel, vw);
 }
@@ -2385,6 +2718,22 @@ __device__ __forceinline__ void rigidContactVelocitiesAt(const Scene &s, uint32_
 __global__ void __launch_bounds__(kThreads) k_rigidContactVelocities(Scene s, uint32_t iterations, Config cfg)
 {
     forEachElem(s.wP, s.N, [&](uint32_t i) { rigidContactVelocitiesAt(s, iterations, cfg, i); });
+}
+
+// The end of a substep without dynamic bodies, fluid or particle-particle contacts in one launch: a
+// particle's velocity, then its contacts' velocity iterations (they read its own velocity alone); the
+// last block copies the predicted bodies into the state, which neither reads.
+__global__ void __launch_bounds__(kThreads) k_finishSubstep(Scene s, float dt, uint32_t contactIterations, Config cfg)
+{
+    pdlEnter();
+    if (blockIdx.x + 1u == gridDim.x) {
+        for (uint32_t b = threadIdx.x; b < s.B; b += blockDim.x) copyPredictedBody(s, b);
+        return;
+    }
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= s.N) return;
+    updateVelocityAt(s, dt, nullptr, i);
+    if (contactIterations) rigidContactVelocitiesAt(s, contactIterations, cfg, i);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -2735,6 +3084,19 @@ void launchRigidPredict(const Scene &s, float dt, float gx, float gy, float gz, 
     k_rigidPredict<<<1, kThreads, 0, st>>>(s, dt, gx, gy, gz);
 }
 
+bool launchPredictWorld(const Scene &s, float dt, const Config &c, cudaStream_t st)
+{
+    if (s.N == 0 || s.wB.tiles || s.nProxy || s.B + s.C > 4u * kThreads) return false;
+    k_predictWorld<<<blocksFor(s.N) + 1u, kThreads, 0, st>>>(s, dt, c.gravity[0], c.gravity[1], c.gravity[2],
+                                                             s.entries != nullptr);
+    return true;
+}
+
+void launchFinishSubstep(const Scene &s, float dt, uint32_t contactIterations, const Config &c, cudaStream_t st)
+{
+    launchPdl(k_finishSubstep, blocksFor(s.N) + 1u, kThreads, st, s, dt, contactIterations, c);
+}
+
 void launchApplyBodyTargets(const Scene &s, const BodyTarget *list, const uint32_t *count, uint32_t capacity,
                             cudaStream_t st)
 {
@@ -2783,6 +3145,10 @@ void launchCellSetup(const Scene &s, uint32_t *scanTmp, void *sortScratch, cudaS
 void launchRigidCandidates(const Scene &s, uint32_t *scanTmp, size_t, cudaStream_t st)
 {
     if (s.N == 0) return;
+    if (!s.wP.tiles && s.N <= kCandidateSmall) {
+        k_rigidCandidatesSmall<<<1, kCandidateBlock, 0, st>>>(s);
+        return;
+    }
     if (s.wP.tiles) cudaMemsetAsync(s.candCount, 0, sizeof(uint32_t) * s.N, st); // scenes not stepped: none
     k_rigidCandidates<false><<<gridFor(s.wP, s.N), kThreads, 0, st>>>(s, nullptr);
     uint32_t *total = scanTmp;
@@ -3247,6 +3613,168 @@ __global__ void __launch_bounds__(kBatchFusedThreads, 2) k_batchFusedIterations(
     }
 }
 
+// ------------------------------------------------------------------------------------------
+// Resident coloured iterations: one CTA runs every iteration of a substep of a coloured schedule with
+// the scene's positions (and colour Jacobi's sums) in shared memory, a block barrier per colour.  A
+// colour of a small scene has fewer constraints than the CTA has threads, so a launch per colour is all
+// latency; here the next colour's records load while the current one is solved.  Per constraint the
+// same device functions, colours in the same order.
+// ------------------------------------------------------------------------------------------
+constexpr uint32_t kColourThreads = 512u;
+
+// An edge or tet in colour order as the resident kernel holds it in shared memory: its particles
+// (16 bits each), rest value, scaled compliance (< 0: disabled) and lambda.
+struct ColourEdge {
+    uint32_t ab;
+    float rest, alpha, lambda;
+};
+struct ColourTet {
+    uint32_t ab, cd;
+    float rest, alpha, lambda;
+};
+
+// One family's colours from its packed records; moves the corrections into x or the sums.
+template <uint32_t kFam, bool kGaussSeidel, class Packed>
+__device__ __forceinline__ void residentColours(const Scene &s, float relax, const uint32_t *starts, uint32_t colours,
+                                                float4 *x, float4 *acc, Packed *records, bool keep)
+{
+    const uint32_t tid = threadIdx.x;
+    auto move = [&](uint32_t i, f3 c) {
+        if constexpr (kGaussSeidel) {
+            const float4 q = x[i];
+            if (q.w > kEps) x[i] = mk4(xyz(q) + c, q.w);
+        } else {
+            acc[i] = mk4(xyz(acc[i]) + c, 0.0f);
+        }
+    };
+    uint32_t begin = starts[0];
+    for (uint32_t k = 0; k < colours; ++k) {
+        const uint32_t end = starts[k + 1u];
+        for (uint32_t q = begin + tid; q < end; q += kColourThreads) {
+            const Packed r = records[q];
+            float next = r.lambda;
+            const uint32_t a = r.ab & 0xffffu, b = r.ab >> 16;
+            if constexpr (kFam == kFamEdges) {
+                f3 cA{0.f, 0.f, 0.f}, cB = cA;
+                if (!(r.alpha < 0.0f)) edgeCorrect(x[a], x[b], r.rest, r.alpha, relax, r.lambda, next, cA, cB);
+                records[q].lambda = next;
+                move(a, cA);
+                move(b, cB);
+            } else {
+                const uint32_t i[4] = {a, b, r.cd & 0xffffu, r.cd >> 16};
+                f3 c[4];
+                const bool solved = tetCorrect(x[i[0]], x[i[1]], x[i[2]], x[i[3]], r.rest, r.alpha, relax, r.lambda, next, c);
+                records[q].lambda = next;
+                if (!solved || r.alpha <= kEps || keep) { // as tileTet
+                    float4 *rec = s.tetRecC + 4 * size_t(q);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        if (solved) rec[j] = mk4(c[j], 0.0f);
+                        else c[j] = xyz(rec[j]);
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) move(i[j], c[j]);
+            }
+        }
+        begin = end;
+        __syncthreads();
+    }
+}
+
+// What a resident coloured kernel holds beside the positions.
+struct ColourResident {
+    ColourEdge *edges;
+    ColourTet *tets;
+    uint32_t *starts; // edges' colour starts, then the tets'
+};
+
+template <uint32_t kFam, bool kGaussSeidel>
+__device__ __forceinline__ void residentFamily(const Scene &s, float dt, float relax, const FusedPlan &plan,
+                                               const ColourResident &r, bool keep)
+{
+    const uint32_t colours = plan.colours[kFam];
+    if (familySize(s, kFam) == 0u || colours == 0u) return;
+    if constexpr (kFam == kFamEdges) {
+        residentColours<kFam, kGaussSeidel>(s, relax, r.starts, colours, s.x, s.softAcc, r.edges, keep);
+    } else if constexpr (kFam == kFamTets) {
+        residentColours<kFam, kGaussSeidel>(s, relax, r.starts + plan.colours[kFamEdges] + 1u, colours, s.x, s.softAcc, r.tets, keep);
+    } else {
+        const uint32_t *starts = plan.starts[kFam];
+        for (uint32_t k = 0; k < colours; ++k) {
+            const uint32_t b = starts[k], e = starts[k + 1];
+            for (uint32_t q = b + threadIdx.x; q < e; q += kColourThreads) colourAt<kFam>(s, dt, relax, kGaussSeidel, q);
+            __syncthreads();
+        }
+    }
+    if constexpr (!kGaussSeidel) {
+        if constexpr (kFam == kFamJoints) {
+            for (uint32_t g = threadIdx.x; g < s.S; g += kColourThreads) colourJacobiOrientAt(s, g);
+        } else {
+            const uint2 win = familyWindow(s, kFam);
+            for (uint32_t i = win.x + threadIdx.x; i < win.y; i += kColourThreads) colourJacobiApplyAt(s, i);
+        }
+        __syncthreads();
+    }
+}
+
+template <bool kGaussSeidel>
+__global__ void __launch_bounds__(kColourThreads, 1) k_residentColour(Scene s, Config cfg, float dt, FusedPlan plan)
+{
+    extern __shared__ float4 tilePos[];
+    // the device functions find the positions and the sums through the scene
+    float4 *global = s.x;
+    s.x = tilePos;
+    if (!kGaussSeidel) s.softAcc = tilePos + s.N;
+    ColourResident r;
+    r.edges = reinterpret_cast<ColourEdge *>(tilePos + (kGaussSeidel ? 1u : 2u) * size_t(s.N));
+    r.tets = reinterpret_cast<ColourTet *>(r.edges + s.E);
+    r.starts = reinterpret_cast<uint32_t *>(r.tets + s.T);
+    const uint32_t tid = threadIdx.x;
+    for (uint32_t i = tid; i < s.N; i += kColourThreads) {
+        s.x[i] = global[i];
+        if (!kGaussSeidel) s.softAcc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    for (uint32_t q = tid; q < s.E; q += kColourThreads) {
+        const PackedEdge e = s.edgesC[q];
+        r.edges[q] = ColourEdge{e.a | (e.b << 16), e.rest, (e.b >> 31) ? -1.0f : scaledCompliance(e.compliance, dt), 0.0f};
+    }
+    for (uint32_t q = tid; q < s.T; q += kColourThreads) {
+        const cn_soft_tet t = s.tetsC[q];
+        r.tets[q] = ColourTet{t.particle_indices[0] | (t.particle_indices[1] << 16),
+                              t.particle_indices[2] | (t.particle_indices[3] << 16), t.rest_volume,
+                              scaledCompliance(t.compliance, dt), 0.0f};
+    }
+    if (s.E)
+        for (uint32_t k = tid; k <= plan.colours[kFamEdges]; k += kColourThreads) r.starts[k] = plan.starts[kFamEdges][k];
+    if (s.T)
+        for (uint32_t k = tid; k <= plan.colours[kFamTets]; k += kColourThreads)
+            r.starts[plan.colours[kFamEdges] + 1u + k] = plan.starts[kFamTets][k];
+    __syncthreads();
+    const float relax = cfg.softInternalRelaxation;
+    for (uint32_t it = 0; it < plan.iterations; ++it) {
+        if (it < plan.softIterations) {
+            const bool keep = it + 1u == plan.softIterations;
+            residentFamily<kFamEdges, kGaussSeidel>(s, dt, relax, plan, r, keep);
+            residentFamily<kFamSegments, kGaussSeidel>(s, dt, relax, plan, r, keep);
+            residentFamily<kFamBends, kGaussSeidel>(s, dt, relax, plan, r, keep);
+            residentFamily<kFamJoints, kGaussSeidel>(s, dt, relax, plan, r, keep);
+            residentFamily<kFamDistances, kGaussSeidel>(s, dt, relax, plan, r, keep);
+            residentFamily<kFamTets, kGaussSeidel>(s, dt, relax, plan, r, keep);
+        }
+        if (plan.rigid != 0u && it < plan.contactIterations) {
+            for (uint32_t i = tid; i < s.N; i += kColourThreads) {
+                const float4 x = s.x[i];
+                bool any;
+                const f3 corr = rigidContactsSum(s, cfg, i, x, contactRange(s, i), it + 1u == plan.contactIterations, any);
+                if (x.w > kEps) s.x[i] = mk4(xyz(x) + corr, x.w);
+            }
+            __syncthreads();
+        }
+    }
+    for (uint32_t i = tid; i < s.N; i += kColourThreads) global[i] = s.x[i];
+}
+
 template <uint32_t kSchedule> cudaError_t fusedLaunch(const Scene &s, const Config &c, float dt, const FusedPlan &plan,
                                                      const FusedShape &shape, cudaStream_t st)
 {
@@ -3273,9 +3801,9 @@ inline unsigned applyGrid(const Scene &s, uint2 win)
 
 
 bool launchSoftIteration(const Scene &s, float dt, const Config &c, const XpbdPlan &plan, cudaStream_t st,
-                         bool rigidContacts)
+                         bool first, bool rigidContacts)
 {
-    if (plan.schedule == CN_XPBD_GATHER) return launchSoftIteration(s, dt, c, st, rigidContacts);
+    if (plan.schedule == CN_XPBD_GATHER) return launchSoftIteration(s, dt, c, st, first, rigidContacts);
     const float relax = c.softInternalRelaxation;
     launchColourFamily<kFamEdges>(s, dt, relax, plan, st);
     launchColourFamily<kFamSegments>(s, dt, relax, plan, st);
@@ -3328,9 +3856,7 @@ FusedShape fusedIterationsShape()
     return out;
 }
 
-void launchFusedIterations(const Scene &s, const Config &c, float dt, const XpbdPlan &plan, uint32_t iterations,
-                           uint32_t softIterations, uint32_t contactIterations, bool rigid, const FusedShape &shape,
-                           cudaStream_t st)
+static FusedPlan fusedPlan(const XpbdPlan &plan, uint32_t iterations, uint32_t softIterations, uint32_t contactIterations, bool rigid)
 {
     FusedPlan fp{};
     fp.iterations = iterations;
@@ -3341,6 +3867,40 @@ void launchFusedIterations(const Scene &s, const Config &c, float dt, const Xpbd
         fp.colours[f] = plan.schedule == CN_XPBD_GATHER ? 0u : plan.colours[f];
         fp.starts[f] = plan.devStarts[f];
     }
+    return fp;
+}
+
+static size_t residentColourBytes(const Scene &s, const XpbdPlan &plan)
+{
+    return size_t(s.N) * sizeof(float4) * (plan.schedule == CN_XPBD_COLOUR_JACOBI ? 2u : 1u) + size_t(s.E) * sizeof(ColourEdge) +
+           size_t(s.T) * sizeof(ColourTet) + (size_t(plan.colours[kFamEdges]) + plan.colours[kFamTets] + 2u) * sizeof(uint32_t);
+}
+
+bool residentColourFits(const Scene &s, const XpbdPlan &plan)
+{
+    if (s.N > 0xffffu || residentColourBytes(s, plan) > kResidentSmemCap) return false;
+    for (const void *f : {reinterpret_cast<const void *>(&k_residentColour<true>), reinterpret_cast<const void *>(&k_residentColour<false>)})
+        if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kResidentSmemCap)) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+    return true;
+}
+
+void launchResidentColour(const Scene &s, const Config &c, float dt, const XpbdPlan &plan, uint32_t iterations,
+                          uint32_t softIterations, uint32_t contactIterations, bool rigid, cudaStream_t st)
+{
+    const FusedPlan fp = fusedPlan(plan, iterations, softIterations, contactIterations, rigid);
+    const size_t bytes = residentColourBytes(s, plan);
+    if (plan.schedule == CN_XPBD_COLOUR_GAUSS_SEIDEL) k_residentColour<true><<<1, kColourThreads, bytes, st>>>(s, c, dt, fp);
+    else k_residentColour<false><<<1, kColourThreads, bytes, st>>>(s, c, dt, fp);
+}
+
+void launchFusedIterations(const Scene &s, const Config &c, float dt, const XpbdPlan &plan, uint32_t iterations,
+                           uint32_t softIterations, uint32_t contactIterations, bool rigid, const FusedShape &shape,
+                           cudaStream_t st)
+{
+    const FusedPlan fp = fusedPlan(plan, iterations, softIterations, contactIterations, rigid);
     if (plan.schedule == CN_XPBD_COLOUR_JACOBI) fusedLaunch<CN_XPBD_COLOUR_JACOBI>(s, c, dt, fp, shape, st);
     else if (plan.schedule == CN_XPBD_COLOUR_GAUSS_SEIDEL) fusedLaunch<CN_XPBD_COLOUR_GAUSS_SEIDEL>(s, c, dt, fp, shape, st);
     else fusedLaunch<CN_XPBD_GATHER>(s, c, dt, fp, shape, st);
@@ -3557,18 +4117,18 @@ void launchBatchFusedIterations(const Scene &s, const Config &c, float dt, const
     cudaLaunchKernelEx(&cfg, k_batchFusedIterations, s, c, dt, plan);
 }
 
-bool launchSoftIteration(const Scene &s, float dt, const Config &c, cudaStream_t st, bool rigidContacts)
+bool launchSoftIteration(const Scene &s, float dt, const Config &c, cudaStream_t st, bool first, bool rigidContacts)
 {
-    return launchSoftFamilies(s, dt, c, st, kAllFamilies, rigidContacts);
+    return launchSoftFamilies(s, dt, c, st, kAllFamilies, first, rigidContacts);
 }
 
-bool launchSoftFamilies(const Scene &s, float dt, const Config &c, cudaStream_t st, uint32_t families,
+bool launchSoftFamilies(const Scene &s, float dt, const Config &c, cudaStream_t st, uint32_t families, bool first,
                         bool rigidContacts)
 {
     const float relax = c.softInternalRelaxation;
     auto on = [&](uint32_t f) { return ((families >> f) & 1u) != 0u; };
     if (s.E && on(kFamEdges)) {
-        launchPdl(k_solveEdges, softGridFor(s.wE, s.E), softThreads(s), st, s, dt, relax);
+        launchPdl(k_solveEdges, softGridFor(s.wE, s.E), softThreads(s), st, s, dt, relax, first);
         launchPdl(k_applyGather, softApplyGrid(s, s.edgeWin), softThreads(s), st, s, s.edgeRanges, s.edgeCorr, s.edgeWin);
     }
     if (s.S && on(kFamSegments)) {
@@ -3589,14 +4149,271 @@ bool launchSoftFamilies(const Scene &s, float dt, const Config &c, cudaStream_t 
         launchPdl(k_applyGather, softApplyGrid(s, s.segWin), softThreads(s), st, s, s.segRanges, s.distCorr, s.segWin);
     }
     if (s.T && on(kFamTets)) {
-        launchPdl(k_solveTets, softGridFor(s.wT, s.T), softThreads(s), st, s, dt, relax);
+        launchPdl(k_solveTets, softGridFor(s.wT, s.T), softThreads(s), st, s, dt, relax, first);
         if (rigidContacts && s.N) {
-            launchPdl(k_applyTetsRigidContacts, softGridFor(s.wP, s.N), softThreads(s), st, s, c);
+            launchPdl(k_applyTetsRigidContacts, softGridFor(s.wP, size_t(s.N) * kGatherLanes), softThreads(s), st, s, c);
             return true;
         }
         launchPdl(k_applyGather, softApplyGrid(s, s.tetWin), softThreads(s), st, s, s.tetRanges, s.tetCorr, s.tetWin);
     }
     return false;
+}
+
+// ------------------------------------------------------------------------------------------
+// Tiled soft iteration
+// ------------------------------------------------------------------------------------------
+namespace {
+
+// One CTA per tile, two on an SM (the contacts' registers; 3 or 4 a SM spill and measured 4-14 % slower).
+// What bounds a stage: a small scene, the chain wait -> positions -> solve (some 250 dependent
+// instructions for a tet) -> sum -> store; a large one, the same chain over too few warps (ncu, 100K
+// particles: issue 43 %, long scoreboard 7.4 per issue, DRAM 13-20 % of peak).  Against the four per-family
+// launches an iteration it saves the correction records' trips through L2 (128 B a tet, 64 B an edge,
+// scattered) and two launches: 100K particles 3.97 -> 2.29 ms a frame of 80 iterations, a cloth of 12.5K
+// 1.29 -> 0.82 ms, 216 particles on the ground 1.24 -> 0.6 ms.
+constexpr int kTileThreads = 256;
+constexpr int kTileBlocks = 2;
+constexpr int kTileAhead = 3;      // entries per thread loaded before the predecessor is waited for
+
+// Per entry: the rest value and the scaled compliance of its constraint record.
+__global__ void __launch_bounds__(kThreads) k_tilePrepare(Scene s, TileSet t, float dt)
+{
+    const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e < t.entries[0]) {
+        const cn_soft_edge &ed = s.edges[t.id[0][e]];
+        t.ra[0][e] = make_float2(ed.rest_length, ed.enabled ? scaledCompliance(ed.compliance, dt) : -1.0f);
+    }
+}
+// The second stage's entries, tile by tile (a tile holds tets, or bends and dihedrals).
+__global__ void __launch_bounds__(kTileThreads) k_tilePrepareElems(Scene s, TileSet t, float dt)
+{
+    const TileHead &h = t.heads[blockIdx.x];
+    const uint32_t end = h.entry[1] + h.entryCount[1];
+    for (uint32_t e = h.entry[1] + threadIdx.x; e < end; e += blockDim.x) {
+        const uint32_t c = t.id[1][e];
+        float rest, compliance;
+        if (!h.bends) {
+            rest = s.tets[c].rest_volume;
+            compliance = s.tets[c].compliance;
+        } else if (c < s.Bn) {
+            rest = s.bends[c].rest_angle;
+            compliance = s.bends[c].compliance;
+        } else {
+            rest = s.dihedrals[c - s.Bn].rest_angle;
+            compliance = s.dihedrals[c - s.Bn].compliance;
+        }
+        t.ra[1][e] = make_float2(rest, scaledCompliance(compliance, dt));
+    }
+}
+
+// The record slots of a stage in shared memory, one plane per component.
+struct TileRecords {
+    float *x, *y, *z;
+    __device__ __forceinline__ void put(uint32_t slot, f3 v) const
+    {
+        if (slot == kTileNoSlot) return;
+        x[slot] = v.x;
+        y[slot] = v.y;
+        z[slot] = v.z;
+    }
+};
+
+__device__ __forceinline__ float tileEdge(const float4 *pos, const TileRecords &rec, uint2 w, float2 ra, float relax,
+                                          float lambda)
+{
+    f3 a{0.f, 0.f, 0.f}, b = a;
+    float next = lambda;
+    if (!(ra.y < 0.0f)) edgeCorrect(pos[w.x & 0xffffu], pos[w.x >> 16], ra.x, ra.y, relax, lambda, next, a, b);
+    rec.put(w.y & 0xffffu, a);
+    rec.put(w.y >> 16, b);
+    return next;
+}
+
+// A tet that cannot be projected keeps its previous corrections (physics_soft_solve_tet_constraints):
+// that takes a scaled compliance of at most kEps, so those tets keep their records in memory; `keep` (the
+// substep's last iteration) stores every tet's, for a compliance that is set to zero between frames.
+__device__ __forceinline__ float tileTet(const Scene &s, const uint32_t *id, const float4 *pos, const TileRecords &rec,
+                                         uint4 w, float2 ra, float relax, float lambda, bool keep)
+{
+    const uint32_t slot[4] = {w.z & 0xffffu, w.z >> 16, w.w & 0xffffu, w.w >> 16};
+    f3 c[4];
+    float next = lambda;
+    const bool solved = tetCorrect(pos[w.x & 0xffffu], pos[w.x >> 16], pos[w.y & 0xffffu], pos[w.y >> 16], ra.x, ra.y,
+                                   relax, lambda, next, c);
+    if (!solved || ra.y <= kEps || keep) {
+        const uint4 d = reinterpret_cast<const uint4 *>(s.tetDst)[*id];
+        const uint32_t dst[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (slot[k] == kTileNoSlot) continue;
+            if (solved) s.tetCorr[dst[k]] = mk4(c[k], 0.0f);
+            else c[k] = xyz(s.tetCorr[dst[k]]);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) rec.put(slot[k], c[k]);
+    return next;
+}
+
+__device__ __forceinline__ float tileBend(const Scene &s, uint32_t id, const float4 *pos, const TileRecords &rec, uint4 w,
+                                          float2 ra, float relax, float lambda)
+{
+    const float4 q0 = pos[w.x & 0xffffu], q1 = pos[w.x >> 16], q2 = pos[w.y & 0xffffu], q3 = pos[w.y >> 16];
+    f3 c[4];
+    c[3] = f3{0.f, 0.f, 0.f};
+    float next = lambda;
+    if (id < s.Bn) bendCorrect(q0, q1, q2, ra.x, ra.y, relax, lambda, next, c);
+    else dihedralCorrect(q0, q1, q2, q3, ra.x, ra.y, relax, lambda, next, c);
+    rec.put(w.z & 0xffffu, c[0]);
+    rec.put(w.z >> 16, c[1]);
+    rec.put(w.w & 0xffffu, c[2]);
+    rec.put(w.w >> 16, c[3]);
+    return next;
+}
+
+template <uint32_t kStage, bool kBends, bool kContacts>
+__global__ void __launch_bounds__(kTileThreads, kTileBlocks) k_tileStage(const __grid_constant__ Scene s, const __grid_constant__ TileSet t,
+                                                               const __grid_constant__ Config cfg, const float4 *xin,
+                                                               float4 *xout, uint32_t tile0, uint32_t flags)
+{
+    extern __shared__ float4 tilePos[];
+    const TileHead h = t.heads[tile0 + blockIdx.x];
+    const uint32_t tid = threadIdx.x, p = h.ownCount, m = p + h.haloCount;
+    const uint32_t e0 = h.entry[kStage], en = h.entryCount[kStage], slots = h.slots[kStage];
+    const bool first = (flags & kTileFirst) != 0u;
+    const float relax = cfg.softInternalRelaxation;
+    float *r0 = reinterpret_cast<float *>(tilePos + m);
+    const TileRecords rec{r0, r0 + slots, r0 + 2 * size_t(slots)};
+    using Words = typename std::conditional<kStage == 0u, uint2, uint4>::type;
+    const Words *words = [&] {
+        if constexpr (kStage == 0u) return t.edges + e0;
+        else return t.elems + e0;
+    }();
+    const uint32_t *ids = t.id[kStage] + e0;
+    const float2 *ra = t.ra[kStage] + e0;
+    float *lambda = t.lambda[kStage] + e0;
+    // Nothing before the wait is written by the stage this one follows: the tile's lists are fixed, the
+    // lambdas are the same stage's of the iteration before, the candidate ranges the substep's.
+    Words w[kTileAhead];
+    float2 c[kTileAhead];
+    float l[kTileAhead];
+#pragma unroll
+    for (int j = 0; j < kTileAhead; ++j) {
+        const uint32_t e = tid + j * kTileThreads;
+        if (e >= en) break;
+        w[j] = words[e];
+        c[j] = ra[e];
+        l[j] = first ? 0.0f : lambda[e];
+    }
+    const uint32_t g0 = tid < p ? t.own[h.own + tid] : (tid < m ? t.halo[h.halo + tid - p] : 0u);
+    const uint32_t j1 = tid + kTileThreads;
+    const uint32_t g1 = j1 < p ? t.own[h.own + j1] : (j1 < m ? t.halo[h.halo + j1 - p] : 0u);
+    ContactRange range{};
+    if (kContacts && tid < p) range = contactRange(s, g0);
+    pdlEnter();
+    if (tid < m) tilePos[tid] = xin[g0];
+    if (j1 < m) tilePos[j1] = xin[g1];
+    for (uint32_t j = tid + 2 * kTileThreads; j < m; j += kTileThreads)
+        tilePos[j] = xin[j < p ? t.own[h.own + j] : t.halo[h.halo + j - p]];
+    __syncthreads();
+    auto solve = [&](uint32_t e, const Words &wd, float2 rc, float lam) {
+        if constexpr (kStage == 0u) lambda[e] = tileEdge(tilePos, rec, wd, rc, relax, lam);
+        else if constexpr (kBends) lambda[e] = tileBend(s, ids[e], tilePos, rec, wd, rc, relax, lam);
+        else lambda[e] = tileTet(s, ids + e, tilePos, rec, wd, rc, relax, lam, (flags & kTileLast) != 0u);
+    };
+#pragma unroll
+    for (int j = 0; j < kTileAhead; ++j) {
+        const uint32_t e = tid + j * kTileThreads;
+        if (e >= en) break;
+        solve(e, w[j], c[j], l[j]);
+    }
+    for (uint32_t e = tid + kTileAhead * kTileThreads; e < en; e += kTileThreads)
+        solve(e, words[e], ra[e], first ? 0.0f : lambda[e]);
+    __syncthreads();
+    // the gather: one thread per own particle and component, records in ascending constraint order
+    for (uint32_t q = tid; q < 3u * p; q += kTileThreads) {
+        const uint32_t comp = q >= 2u * p ? 2u : (q >= p ? 1u : 0u), i = q - comp * p;
+        if (tilePos[i].w <= kEps) continue;
+        const uint32_t r = t.rec[kStage][h.own + i];
+        const float *src = r0 + comp * size_t(slots) + tileRecordBase(r);
+        const uint32_t width = tileRecordWidth(r), count = tileRecordCount(r);
+        float total = 0.0f;
+#pragma unroll 4
+        for (uint32_t k = 0; k < count; ++k) total += src[k * width];
+        float *x = reinterpret_cast<float *>(tilePos + i) + comp;
+        *x = *x + total;
+    }
+    __syncthreads();
+    for (uint32_t i = tid; i < p; i += kTileThreads) {
+        const uint32_t g = i == tid ? g0 : t.own[h.own + i];
+        const float4 x = tilePos[i];
+        if constexpr (kContacts) {
+            if (i != tid) range = contactRange(s, g);
+            if (range.count) rigidContactsFrom(s, cfg, true, g, x, range); // writes s.x == xout
+            else if (x.w > kEps) xout[g] = mk4(xyz(x) + f3{0.f, 0.f, 0.f}, x.w); // as a particle without contacts
+        } else {
+            xout[g] = x;
+        }
+    }
+}
+
+template <uint32_t kStage, bool kBends, bool kContacts>
+void launchTileStage(const Scene &s, const TileSet &t, const Config &c, const float4 *xin, float4 *xout, uint32_t tile0,
+                     uint32_t tiles, uint32_t flags, cudaStream_t st)
+{
+    if (tiles == 0u) return;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(tiles, 1, 1);
+    cfg.blockDim = dim3(kTileThreads, 1, 1);
+    cfg.dynamicSmemBytes = t.smem[kStage];
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdlEnabled() ? 1u : 0u;
+    cudaLaunchKernelEx(&cfg, k_tileStage<kStage, kBends, kContacts>, s, t, c, xin, xout, tile0, flags);
+}
+
+} // namespace
+
+void launchTilePrepare(const Scene &s, const TileSet &t, float dt, cudaStream_t st)
+{
+    if (t.entries[0]) k_tilePrepare<<<blocksFor(t.entries[0]), kThreads, 0, st>>>(s, t, dt);
+    if (t.entries[1]) k_tilePrepareElems<<<t.tiles, kTileThreads, 0, st>>>(s, t, dt);
+}
+
+void launchTileEdges(const Scene &s, const TileSet &t, const Config &c, uint32_t flags, cudaStream_t st)
+{
+    launchTileStage<0u, false, false>(s, t, c, s.x, t.xB, 0u, t.tiles, flags, st);
+}
+
+void launchTileTets(const Scene &s, const TileSet &t, const Config &c, uint32_t flags, bool contacts, cudaStream_t st)
+{
+    if (contacts) launchTileStage<1u, false, true>(s, t, c, t.xB, s.x, 0u, t.tetTiles, flags, st);
+    else launchTileStage<1u, false, false>(s, t, c, t.xB, s.x, 0u, t.tetTiles, flags, st);
+}
+
+void launchTileBends(const Scene &s, const TileSet &t, const Config &c, uint32_t flags, bool contacts, cudaStream_t st)
+{
+    const uint32_t n = t.tiles - t.tetTiles;
+    if (contacts) launchTileStage<1u, true, true>(s, t, c, t.xB, s.x, t.tetTiles, n, flags, st);
+    else launchTileStage<1u, true, false>(s, t, c, t.xB, s.x, t.tetTiles, n, flags, st);
+}
+
+bool tileKernelsFit(uint32_t bytes)
+{
+    const void *fns[] = {reinterpret_cast<const void *>(&k_tileStage<0u, false, false>),
+                         reinterpret_cast<const void *>(&k_tileStage<1u, true, true>),
+                         reinterpret_cast<const void *>(&k_tileStage<1u, true, false>),
+                         reinterpret_cast<const void *>(&k_tileStage<1u, false, true>),
+                         reinterpret_cast<const void *>(&k_tileStage<1u, false, false>)};
+    for (const void *f : fns)
+        if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+    return true;
 }
 
 void launchContacts(const Scene &s, const Config &c, bool particleContacts, bool rigidContacts,

@@ -19,6 +19,7 @@
 #include "../../include/cn_physics.h"
 #include "cn_device.h"
 #include "cn_internal.h"
+#include "cn_tiles.h"
 
 namespace cn {
 
@@ -89,6 +90,12 @@ struct cn_solver {
     cudaStream_t side[3] = {nullptr, nullptr, nullptr};
     cudaEvent_t fork = nullptr, joinFluid = nullptr, joinStrands = nullptr, afterEdges = nullptr, joinBends = nullptr;
     bool branchFluid = false, branchStrands = false, branchBends = false;
+    // Tiled soft iterations (gather schedule): the tile lists, and whether the particle-rigid
+    // contacts run in the second stage
+    cn::TileBuild tileBuild;
+    cn::TileSet tiles{};
+    bool tileContacts = false;
+    bool residentColour = false; // a coloured schedule's iterations in one CTA
 };
 
 namespace {
@@ -199,6 +206,29 @@ void layout(cn_solver *sv, cn::Arena &a, const cn_world_soa &w, const cn::Incide
     s.distCorr = a.take<float4>(s.SD ? std::max<size_t>(size_t(s.SD) * 2, segI.inc.size()) : 0);
     s.posCorr = a.take<float4>(N);
     s.velCorr = a.take<float4>(N);
+    {
+        const cn::TileBuild &tb = sv->tileBuild;
+        cn::TileSet &t = sv->tiles;
+        t = cn::TileSet{};
+        if (tb.ok) {
+            t.tiles = uint32_t(tb.heads.size());
+            t.heads = a.take<cn::TileHead>(tb.heads.size());
+            t.own = a.take<uint32_t>(tb.own.size());
+            t.halo = a.take<uint32_t>(tb.halo.size());
+            for (int f = 0; f < 2; ++f) {
+                t.entries[f] = uint32_t(tb.id[f].size());
+                t.smem[f] = tb.smem[f];
+                t.rec[f] = a.take<uint32_t>(tb.rec[f].size());
+                t.id[f] = a.take<uint32_t>(tb.id[f].size());
+                t.ra[f] = a.take<float2>(tb.id[f].size());
+                t.lambda[f] = a.take<float>(tb.id[f].size());
+            }
+            t.edges = a.take<uint2>(tb.edges.size());
+            t.elems = a.take<uint4>(tb.elems.size());
+            t.xB = a.take<float4>(N);
+            for (const cn::TileHead &h : tb.heads) t.tetTiles += h.bends ? 0u : 1u;
+        }
+    }
     for (uint32_t f = 0; f < cn::kFamilies; ++f) {
         const cn::Colouring &col = sv->colouring[f];
         s.colOrder[f] = col.colours() ? a.take<uint32_t>(col.order.size()) : nullptr;
@@ -228,6 +258,7 @@ void layout(cn_solver *sv, cn::Arena &a, const cn_world_soa &w, const cn::Incide
     s.prevBodyPos = a.take<float4>(B); s.prevBodyRot = a.take<float4>(B);
     s.predBodyPos = a.take<float4>(B); s.predBodyRot = a.take<float4>(B);
     s.predBodyLin = a.take<float4>(B); s.predBodyAng = a.take<float4>(B);
+    s.prevBodyUnit = a.take<float4>(B); s.predBodyUnit = a.take<float4>(B);
     s.colAabbMin = a.take<float4>(C); s.colAabbMax = a.take<float4>(C);
     s.nProxy = sv->nProxy;
     s.proxyLocal = a.take<float4>(sv->nProxy);
@@ -430,31 +461,46 @@ cn_status uploadSurfaceRender(cn_solver *sv, const cn_world_soa &w, cudaStream_t
     return CN_OK;
 }
 
+constexpr uint32_t kTileFams = (1u << cn::kFamEdges) | (1u << cn::kFamBends) | (1u << cn::kFamTets);
+constexpr uint32_t kStrandFams = (1u << cn::kFamSegments) | (1u << cn::kFamJoints) | (1u << cn::kFamDistances);
+
 // One iteration's soft families with the strand families on a side stream and, once the edges
 // are applied, the cloth bends on another, joined back before the stream goes on (each particle's
 // families still in the order of physics_solver.cpp:915-1019).
-void launchSoftBranches(cn_solver *sv, float dt, cudaStream_t st)
+void launchSoftBranches(cn_solver *sv, float dt, uint32_t flags, cudaStream_t st)
 {
+    const bool first = (flags & cn::kTileFirst) != 0u;
     const cn::Scene &s = sv->s;
     const cn::Config &c = sv->cfg;
-    const uint32_t strandFams = (1u << cn::kFamSegments) | (1u << cn::kFamJoints) | (1u << cn::kFamDistances);
     uint32_t mainFams = cn::kAllFamilies;
     if (sv->branchStrands) {
         cudaStreamWaitEvent(sv->side[1], sv->fork, 0);
-        cn::launchSoftFamilies(s, dt, c, sv->side[1], strandFams);
+        cn::launchSoftFamilies(s, dt, c, sv->side[1], kStrandFams, first);
         cudaEventRecord(sv->joinStrands, sv->side[1]);
-        mainFams &= ~strandFams;
+        mainFams &= ~kStrandFams;
     }
-    if (sv->branchBends) {
-        cn::launchSoftFamilies(s, dt, c, st, mainFams & (1u << cn::kFamEdges));
+    if (sv->tiles.tiles) {
+        cn::launchTileEdges(s, sv->tiles, c, flags, st);
+        const cudaStream_t bst = sv->branchBends ? sv->side[2] : st;
+        if (sv->branchBends) {
+            cudaEventRecord(sv->afterEdges, st);
+            cudaStreamWaitEvent(bst, sv->afterEdges, 0);
+        }
+        cn::launchTileBends(s, sv->tiles, c, flags, false, bst);
+        if (sv->branchBends) cudaEventRecord(sv->joinBends, bst);
+        cn::launchTileTets(s, sv->tiles, c, flags, false, st);
+        if (sv->branchBends) cudaStreamWaitEvent(st, sv->joinBends, 0);
+        cn::launchSoftFamilies(s, dt, c, st, mainFams & ~kTileFams, first);
+    } else if (sv->branchBends) {
+        cn::launchSoftFamilies(s, dt, c, st, mainFams & (1u << cn::kFamEdges), first);
         cudaEventRecord(sv->afterEdges, st);
         cudaStreamWaitEvent(sv->side[2], sv->afterEdges, 0);
-        cn::launchSoftFamilies(s, dt, c, sv->side[2], 1u << cn::kFamBends);
+        cn::launchSoftFamilies(s, dt, c, sv->side[2], 1u << cn::kFamBends, first);
         cudaEventRecord(sv->joinBends, sv->side[2]);
-        cn::launchSoftFamilies(s, dt, c, st, mainFams & ~((1u << cn::kFamEdges) | (1u << cn::kFamBends)));
+        cn::launchSoftFamilies(s, dt, c, st, mainFams & ~((1u << cn::kFamEdges) | (1u << cn::kFamBends)), first);
         cudaStreamWaitEvent(st, sv->joinBends, 0);
     } else {
-        cn::launchSoftFamilies(s, dt, c, st, mainFams);
+        cn::launchSoftFamilies(s, dt, c, st, mainFams, first);
     }
     if (sv->branchStrands) cudaStreamWaitEvent(st, sv->joinStrands, 0);
 }
@@ -465,12 +511,17 @@ void enqueueFrame(cn_solver *sv, float frameDt, cudaStream_t st)
     const float dt = frameDt / float(sv->substeps);
     const cn::Config &c = sv->cfg;
     const uint32_t N = s.N;
+    if (sv->tiles.tiles && !sv->fused) cn::launchTilePrepare(s, sv->tiles, dt, st);
     for (uint32_t sub = 0; sub < sv->substeps; ++sub) {
-        probe(sv, "rigid_predict", st, [&] { cn::launchRigidPredict(s, dt, c.gravity[0], c.gravity[1], c.gravity[2], st); });
+        bool predicted = false;
+        if (!s.colBvh && !sv->rigidRigid && !sv->timing) predicted = cn::launchPredictWorld(s, dt, c, st);
+        if (!predicted)
+            probe(sv, "rigid_predict", st,
+                  [&] { cn::launchRigidPredict(s, dt, c.gravity[0], c.gravity[1], c.gravity[2], st); });
         if (s.colBvh) probe(sv, "collider_bvh", st, [&] { cn::launchColliderBvh(s, sv->rigidScratch, st); });
         if (sv->rigidRigid)
             probe(sv, "rigid_broadphase_contacts", st, [&] { cn::launchRigidBroadphaseAndContacts(s, c, sv->rigidScratch, st); });
-        probe(sv, "predict_keys", st, [&] { cn::launchPredictAndKeys(s, dt, c, st); });
+        if (!predicted) probe(sv, "predict_keys", st, [&] { cn::launchPredictAndKeys(s, dt, c, st); });
         if (sv->hasBroadphase && (sv->hasFluid || sv->ppPossible || sv->forceBroadphase)) {
             probe(sv, "radix_sort", st, [&] {
                 cn::radixSortPairs(s.keysA, s.valsA, s.keysB, s.valsB, N, sv->sortScratch, &s.meta_->waitTimeouts, st);
@@ -486,9 +537,14 @@ void enqueueFrame(cn_solver *sv, float frameDt, cudaStream_t st)
         // initRigidContactVelocities (physics_solver.cpp:736-743)
         if (sv->rigidRigid) cn::launchRigidVelocityInit(s, c, sv->rigidScratch, st);
         // clearSoftConstraintState (physics_clear_soft_constraint_state.cs.hlsl:14-54)
-        if (s.E) cudaMemsetAsync(s.edgeLambda, 0, sizeof(float) * s.E, st);
-        if (s.Bn + s.D) cudaMemsetAsync(s.bendLambda, 0, sizeof(float) * (s.Bn + s.D), st);
-        if (s.T) cudaMemsetAsync(s.tetLambda, 0, sizeof(float) * s.T, st);
+        // (the tiles and the per-phase edge and tet solves start from zero lambdas by themselves)
+        const bool colours = sv->plan.schedule != CN_XPBD_GATHER && !sv->residentColour;
+        if (colours || sv->fused) {
+            if (s.E) cudaMemsetAsync(s.edgeLambda, 0, sizeof(float) * s.E, st);
+            if (s.T) cudaMemsetAsync(s.tetLambda, 0, sizeof(float) * s.T, st);
+        }
+        if (s.Bn + s.D && (!sv->tiles.tiles || sv->fused))
+            cudaMemsetAsync(s.bendLambda, 0, sizeof(float) * (s.Bn + s.D), st);
         if (s.SD) cudaMemsetAsync(s.distLambda, 0, sizeof(float) * s.SD, st);
         if (s.S) cudaMemsetAsync(s.segLambda, 0, sizeof(float4) * s.S, st);
         if (s.J) cudaMemsetAsync(s.jointLambda, 0, sizeof(float4) * s.J, st);
@@ -514,7 +570,16 @@ void enqueueFrame(cn_solver *sv, float frameDt, cudaStream_t st)
                                           sv->rigidPossible, sv->fusedShape, st);
             });
         }
-        for (uint32_t it = 0; it < (sv->fused ? 0u : sv->maxIt); ++it) {
+        const bool resident = !sv->fused && sv->residentColour;
+        if (resident) { // a small scene's coloured iterations in one CTA
+            const uint32_t softIt = hasSoftInternal ? sv->softIt : 0u;
+            const uint32_t contactIt = sv->rigidPossible ? sv->contactIt : 0u;
+            probe(sv, "soft_constraints", st, [&] {
+                cn::launchResidentColour(s, c, dt, sv->plan, std::max(softIt, contactIt), softIt, contactIt,
+                                         sv->rigidPossible, st);
+            });
+        }
+        for (uint32_t it = 0; it < (sv->fused || resident ? 0u : sv->maxIt); ++it) {
             const bool runFluid = sv->hasFluid && it < sv->fluidIt;
             const bool runSoft = hasSoftInternal && it < sv->softIt;
             const bool runPP = sv->ppPossible && it < sv->contactIt;
@@ -542,12 +607,21 @@ void enqueueFrame(cn_solver *sv, float frameDt, cudaStream_t st)
             // contact pass writes them
             cn::Scene si = s;
             si.storeRigidContacts = it + 1 == sv->contactIt ? 1u : 0u;
+            const uint32_t flags = (it == 0 ? cn::kTileFirst : 0u) | (it + 1 == sv->softIt ? cn::kTileLast : 0u);
             bool contactsDone = false;
             if (runSoft && softBranches)
-                probe(sv, "soft_constraints", st, [&] { launchSoftBranches(sv, dt, st); });
+                probe(sv, "soft_constraints", st, [&] { launchSoftBranches(sv, dt, flags, st); });
+            else if (runSoft && sv->tiles.tiles)
+                probe(sv, "soft_constraints", st, [&] {
+                    contactsDone = sv->tileContacts && runRigid && !runPP;
+                    cn::launchTileEdges(si, sv->tiles, c, flags, st);
+                    cn::launchTileTets(si, sv->tiles, c, flags, contactsDone, st);
+                    cn::launchTileBends(si, sv->tiles, c, flags, contactsDone, st);
+                    cn::launchSoftFamilies(si, dt, c, st, kStrandFams, it == 0); // on particles of their own
+                });
             else if (runSoft)
                 probe(sv, "soft_constraints", st, [&] {
-                    contactsDone = cn::launchSoftIteration(si, dt, c, sv->plan, st, runRigid && !runPP);
+                    contactsDone = cn::launchSoftIteration(si, dt, c, sv->plan, st, it == 0, runRigid && !runPP);
                 });
             if (fluidBranch) cudaStreamWaitEvent(st, sv->joinFluid, 0);
             if ((runPP || runRigid) && !contactsDone)
@@ -564,6 +638,10 @@ void enqueueFrame(cn_solver *sv, float frameDt, cudaStream_t st)
         // updateRigidVelocities (physics_solver.cpp:1241-1246): for static and kinematic bodies it
         // restates what the rigid predict wrote, so it runs for scenes with dynamic bodies
         if (s.hasDynamic) cn::launchUpdateRigidVelocities(s, dt, st);
+        if (N > 0 && !s.hasDynamic && !sv->hasFluid && !sv->ppPossible && !sv->timing) {
+            cn::launchFinishSubstep(s, dt, sv->rigidPossible ? sv->contactIt : 0u, c, st);
+            continue;
+        }
         const float4 *fluidDelta = sv->hasFluid ? ((sv->fluidIt & 1u) ? s.Db : s.Da) : nullptr;
         probe(sv, "update_velocities", st, [&] { cn::launchUpdateVelocities(s, dt, fluidDelta, st); });
         if (sv->hasFluid) probe(sv, "fluid_boundary_velocities", st, [&] { cn::launchFluidBoundaryVelocities(s, dt, c, st); });
@@ -772,6 +850,69 @@ static cudaError_t uploadColourOrdered(cn_solver *sv, const cn_world_soa &w, cud
     return cudaSuccess;
 }
 
+// Every constraint names particles (segments) of the world: what the tiled and the resident iterations
+// require, whose positions sit in shared memory.
+static bool constraintIndicesValid(const cn_world_soa &w)
+{
+    const uint32_t N = w.particle_count, S = w.strand_segment_count;
+    bool ok = true;
+    for (uint32_t c = 0; c < w.edge_count; ++c) ok &= w.edges[c].particle_a < N && w.edges[c].particle_b < N;
+    for (uint32_t c = 0; c < w.tet_count; ++c)
+        for (uint32_t p : w.tets[c].particle_indices) ok &= p < N;
+    for (uint32_t c = 0; c < w.bend_count; ++c)
+        ok &= w.bends[c].particle0 < N && w.bends[c].particle1 < N && w.bends[c].particle2 < N;
+    for (uint32_t c = 0; c < w.dihedral_count; ++c) {
+        const cn_cloth_dihedral &h = w.dihedrals[c];
+        ok &= h.edge_particle0 < N && h.edge_particle1 < N && h.opposite_particle0 < N && h.opposite_particle1 < N;
+    }
+    for (uint32_t c = 0; c < S; ++c) ok &= w.strand_segments[c].particle_a < N && w.strand_segments[c].particle_b < N;
+    for (uint32_t c = 0; c < w.strand_joint_count; ++c)
+        ok &= w.strand_joints[c].segment_a < S && w.strand_joints[c].segment_b < S;
+    for (uint32_t c = 0; c < w.strand_distance_count; ++c)
+        ok &= w.strand_distances[c].particle_a < N && w.strand_distances[c].particle_b < N;
+    return ok;
+}
+
+// Cuts the soft families of a world into tiles.  Taken by the gather schedule where every particle
+// of the tiles sees its families in two stages: edges, then tets or bends (a particle of both keeps the
+// per-family kernels), strands on particles of their own.
+static void buildSolverTiles(cn_solver *sv, const cn_world_soa &w, const cn::Incidence &edgeI, const cn::Incidence &bendI,
+                             const cn::Incidence &tetI, const cn::Incidence &segI)
+{
+    sv->tileBuild = cn::TileBuild{};
+    sv->tileContacts = false;
+    const uint32_t N = w.particle_count;
+    if (sv->plan.schedule != CN_XPBD_GATHER || sv->desc.soft.fused_iterations != CN_FUSED_OFF) return;
+    if (N == 0 || !(w.edge_count || w.tet_count || w.bend_count || w.dihedral_count)) return;
+    const uint32_t nb = w.bend_count;
+    auto edgeOf = [&](uint32_t c, uint32_t k) { return k == 0 ? w.edges[c].particle_a : w.edges[c].particle_b; };
+    auto tetOf = [&](uint32_t c, uint32_t k) { return w.tets[c].particle_indices[k]; };
+    auto bendOf = [&](uint32_t c, uint32_t k) -> uint32_t {
+        if (c < nb) return k == 0 ? w.bends[c].particle0 : k == 1 ? w.bends[c].particle1 : k == 2 ? w.bends[c].particle2 : N;
+        const cn_cloth_dihedral &h = w.dihedrals[c - nb];
+        return k == 0 ? h.edge_particle0 : k == 1 ? h.edge_particle1 : k == 2 ? h.opposite_particle0 : h.opposite_particle1;
+    };
+    if (!constraintIndicesValid(w)) return;
+    // the contacts of every particle run in the second stage when nothing else moves particles between
+    const bool strands = w.strand_segment_count || w.strand_joint_count || w.strand_distance_count;
+    const bool contacts = sv->rigidPossible && !sv->ppPossible && !sv->hasFluid && !strands;
+    std::vector<uint8_t> cls(N, 0);
+    for (uint32_t i = 0; i < N; ++i) {
+        const bool t = tetI.ranges[i].y != 0, b = bendI.ranges[i].y != 0;
+        if (t && b) return;
+        const bool any = t || b || edgeI.ranges[i].y != 0;
+        if (any && segI.ranges[i].y != 0) return;
+        if (any || contacts) cls[i] = b ? 2 : 1;
+    }
+    using In = cn::TileInput<decltype(edgeOf), decltype(tetOf), decltype(bendOf)>;
+    const In in{N, w.positions_inv_mass, cls, edgeI, tetI, bendI, edgeOf, tetOf, bendOf};
+    sv->tileContacts = contacts;
+    const uint32_t target = cn::tileTarget(N);
+    if (!target) return;
+    sv->tileBuild = cn::buildTiles(in, target, cn::kTileSmemCap);
+    if (sv->tileBuild.ok && !cn::tileKernelsFit(cn::kTileSmemCap)) sv->tileBuild = cn::TileBuild{};
+}
+
 CN_API cn_status cn_solver_sync_world(cn_solver *sv, const cn_world_soa *w)
 {
     if (!sv || !w) return setError(CN_ERR_INVALID_ARGUMENT, "cn_solver_sync_world: null argument");
@@ -971,6 +1112,8 @@ CN_API cn_status cn_solver_sync_world(cn_solver *sv, const cn_world_soa *w)
         }
     }
 
+    buildSolverTiles(sv, *w, edgeI, bendI, tetI, segI);
+
     cn::Arena a;
     a.reset(nullptr);
     layout(sv, a, *w, edgeI, bendI, tetI, segI, jointI);
@@ -1062,6 +1205,19 @@ CN_API cn_status cn_solver_sync_world(cn_solver *sv, const cn_world_soa *w)
         CN_CUDA(up(const_cast<uint32_t *>(sv->plan.devStarts[f]), col.starts.data(), col.starts.size(), st));
     }
     CN_CUDA(uploadColourOrdered(sv, *w, st));
+    if (sv->tiles.tiles) {
+        const cn::TileBuild &tb = sv->tileBuild;
+        const cn::TileSet &t = sv->tiles;
+        CN_CUDA(up(t.heads, tb.heads.data(), tb.heads.size(), st));
+        CN_CUDA(up(t.own, tb.own.data(), tb.own.size(), st));
+        CN_CUDA(up(t.halo, tb.halo.data(), tb.halo.size(), st));
+        for (int f = 0; f < 2; ++f) {
+            CN_CUDA(up(t.rec[f], tb.rec[f].data(), tb.rec[f].size(), st));
+            CN_CUDA(up(t.id[f], tb.id[f].data(), tb.id[f].size(), st));
+        }
+        CN_CUDA(up(t.edges, tb.edges.data(), tb.edges.size(), st));
+        CN_CUDA(up(t.elems, tb.elems.data(), tb.elems.size(), st));
+    }
     CN_CUDA(up(s.bodyPos, w->body_positions_inv_mass, s.B, st));
     CN_CUDA(up(s.bodyRot, w->body_orientations, s.B, st));
     CN_CUDA(up(s.bodyLin, w->body_linear_velocities, s.B, st));
@@ -1104,6 +1260,12 @@ CN_API cn_status cn_solver_sync_world(cn_solver *sv, const cn_world_soa *w)
                                         uint64_t(s.J), uint64_t(s.SD)});
         sv->fused = cap > 0 && most <= cap;
     }
+    // Coloured iterations in one CTA: the conditions of the fused ones, the positions in shared memory
+    sv->residentColour = !sv->fused && sv->plan.schedule != CN_XPBD_GATHER && N > 0 && !sv->hasFluid && !sv->ppPossible &&
+                         !sv->hasDynamic && !sv->rigidRigid && nProxy == 0 &&
+                         (s.E || s.Bn || s.D || s.T || s.S || s.J || s.SD) &&
+                         constraintIndicesValid(*w) &&
+                         cn::residentColourFits(s, sv->plan);
     // Concurrent branches (per-phase gather schedule): the strand families beside the others, the
     // cloth bends beside the tets once the edges are applied, and the fluid chain beside the soft
     // families, whenever the particle windows they write are disjoint.
@@ -1125,6 +1287,7 @@ CN_API cn_status cn_solver_sync_world(cn_solver *sv, const cn_world_soa *w)
                           disjoint(fluidWin, s.bendWin) && disjoint(fluidWin, s.tetWin) &&
                           disjoint(fluidWin, s.segWin);
     }
+    sv->tileBuild = cn::TileBuild{}; // uploaded
     sv->hostX = w->positions_inv_mass;
     sv->hostV = w->velocities;
     sv->contactMaterialCapacity = w->contact_material_count;
