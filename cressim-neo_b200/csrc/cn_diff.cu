@@ -8,13 +8,15 @@
 // (k_predictKeys, k_solveEdges, k_applyPair, k_solveTets, k_applyQuad, k_updateVelocities)
 // expression for expression, so in float it reproduces their bits.
 //
-// The adjoint runs the iterations backwards: per constraint, the Jacobian of (corrections,
-// lambda') with respect to (positions, lambda, compliance) comes from the same templated
-// constraint code evaluated on forward-mode dual numbers, and the vector-Jacobian products are
-// written as per-constraint records that each particle gathers in ascending constraint order
-// (deterministic, no atomics).  Positions and velocities are checkpointed at the start of every
+// The adjoint runs the iterations backwards: per constraint, the vector-Jacobian product of
+// (corrections, lambda') with respect to (positions, lambda, compliance) is written out in reverse
+// (edgeAdjoint, tetAdjoint; about twice the forward's operations, where tangents of every input
+// would take 7 and 14 times as many), and goes to records that each particle gathers in ascending
+// constraint order (deterministic, no atomics).  Positions and velocities are checkpointed at the start of every
 // `checkpoint_interval`-th substep; backward recomputes one segment of substeps from its
-// checkpoint, then one substep's iteration states at a time.
+// checkpoint, then one substep's iteration states at a time.  A substep and a substep's adjoint are
+// each one CUDA graph, captured at first use (the launches of 8 substeps x 20 iterations took the host
+// longer than the device).
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -33,79 +35,11 @@ namespace {
 constexpr int kDiffThreads = 256;
 inline unsigned gridOf(size_t n) { return n == 0 ? 1u : unsigned((n + kDiffThreads - 1) / kDiffThreads); }
 
-// ---------------------------------------------------------------- scalar types
-// A value with K tangents (forward mode).  Only the operations the constraint code uses.
-template <class T, int K> struct Dual {
-    T v;
-    T d[K];
-};
-template <class T> __host__ __device__ __forceinline__ T val(T x) { return x; }
-template <class T, int K> __host__ __device__ __forceinline__ T val(const Dual<T, K> &x) { return x.v; }
-
-template <class T, int K> __device__ __forceinline__ Dual<T, K> mkc(T c)
-{
-    Dual<T, K> r;
-    r.v = c;
-#pragma unroll
-    for (int k = 0; k < K; ++k) r.d[k] = T(0);
-    return r;
-}
-template <class T, int K> __device__ __forceinline__ Dual<T, K> operator+(const Dual<T, K> &a, const Dual<T, K> &b)
-{
-    Dual<T, K> r;
-    r.v = a.v + b.v;
-#pragma unroll
-    for (int k = 0; k < K; ++k) r.d[k] = a.d[k] + b.d[k];
-    return r;
-}
-template <class T, int K> __device__ __forceinline__ Dual<T, K> operator-(const Dual<T, K> &a, const Dual<T, K> &b)
-{
-    Dual<T, K> r;
-    r.v = a.v - b.v;
-#pragma unroll
-    for (int k = 0; k < K; ++k) r.d[k] = a.d[k] - b.d[k];
-    return r;
-}
-template <class T, int K> __device__ __forceinline__ Dual<T, K> operator-(const Dual<T, K> &a)
-{
-    Dual<T, K> r;
-    r.v = -a.v;
-#pragma unroll
-    for (int k = 0; k < K; ++k) r.d[k] = -a.d[k];
-    return r;
-}
-template <class T, int K> __device__ __forceinline__ Dual<T, K> operator*(const Dual<T, K> &a, const Dual<T, K> &b)
-{
-    Dual<T, K> r;
-    r.v = a.v * b.v;
-#pragma unroll
-    for (int k = 0; k < K; ++k) r.d[k] = a.d[k] * b.v + a.v * b.d[k];
-    return r;
-}
-template <class T, int K> __device__ __forceinline__ Dual<T, K> operator/(const Dual<T, K> &a, const Dual<T, K> &b)
-{
-    Dual<T, K> r;
-    r.v = a.v / b.v;
-    const T inv = T(1) / b.v;
-#pragma unroll
-    for (int k = 0; k < K; ++k) r.d[k] = (a.d[k] - r.v * b.d[k]) * inv;
-    return r;
-}
-template <class T, int K> __device__ __forceinline__ Dual<T, K> sqrtD(const Dual<T, K> &a)
-{
-    Dual<T, K> r;
-    r.v = sqrt(a.v);
-    const T h = T(0.5) / r.v;
-#pragma unroll
-    for (int k = 0; k < K; ++k) r.d[k] = a.d[k] * h;
-    return r;
-}
+// ---------------------------------------------------------------- vectors
 __device__ __forceinline__ float sqrtD(float a) { return sqrtf(a); }
 __device__ __forceinline__ double sqrtD(double a) { return sqrt(a); }
-
-// a scalar constant of the same type as `like`
-template <class T> __device__ __forceinline__ T cst(T, double c) { return T(c); }
-template <class T, int K> __device__ __forceinline__ Dual<T, K> cst(const Dual<T, K> &, double c) { return mkc<T, K>(T(c)); }
+__device__ __forceinline__ float absD(float a) { return fabsf(a); }
+__device__ __forceinline__ double absD(double a) { return fabs(a); }
 
 template <class S> struct V3 {
     S x, y, z;
@@ -127,73 +61,123 @@ template <class T> struct P4 {
 };
 
 // ---------------------------------------------------------------- constraint math
-// physics_soft_solve_edge_constraints.cs.hlsl:10-74 (k_solveEdges).  Returns false when the
-// record is written as zeros (disabled, no mass, zero length, no denominator): then lambda' = lambda.
-template <class S, class T>
-__device__ __forceinline__ bool edgeProject(const V3<S> &a, const V3<S> &b, T wA, T wB, T rest, const S &compliance,
-                                            const S &lambda, T dt, T relax, V3<S> &cA, V3<S> &cB, S &lambdaOut)
+// physics_soft_solve_edge_constraints.cs.hlsl:10-74 (k_solveEdges): what the forward and the adjoint share.
+// False when the record is written as zeros (no mass, zero length, no denominator): then lambda' = lambda.
+template <class T> struct EdgeTerms {
+    V3<T> delta;
+    T len, alpha, den, dl;
+};
+template <class T>
+__device__ __forceinline__ bool edgeTerms(const V3<T> &a, const V3<T> &b, T wA, T wB, T rest, T compliance, T lambda, T dt,
+                                          EdgeTerms<T> &e)
 {
     const T eps = T(1.0e-6);
     const T wSum = wA + wB;
-    const V3<S> delta = b - a;
-    const S l2 = dot3(delta, delta);
-    lambdaOut = lambda;
-    if (!(wSum > eps && val(l2) > eps)) return false;
-    const S len = sqrtD(l2);
-    const V3<S> gA = (-delta) / len;
-    const V3<S> gB = -gA;
+    e.delta = b - a;
+    const T l2 = dot3(e.delta, e.delta);
+    if (!(wSum > eps && l2 > eps)) return false;
+    e.len = sqrtD(l2);
     const T dt2 = dt * dt;
-    const S alpha = compliance / cst(l2, dt2 > eps ? dt2 : eps); // max(compliance, 0): compliance > 0 here
-    const S Cv = len - cst(l2, rest);
-    const S den = cst(l2, wSum) + alpha;
-    if (!(val(den) > eps)) return false;
-    const S dl = -(Cv + alpha * lambda) / den;
-    lambdaOut = lambda + dl;
-    cA = ((cst(l2, wA) * dl) * gA) * cst(l2, relax);
-    cB = ((cst(l2, wB) * dl) * gB) * cst(l2, relax);
+    e.alpha = compliance / (dt2 > eps ? dt2 : eps); // max(compliance, 0): compliance > 0 here
+    const T Cv = e.len - rest;
+    e.den = wSum + e.alpha;
+    if (!(e.den > eps)) return false;
+    e.dl = -(Cv + e.alpha * lambda) / e.den;
     return true;
 }
 
-// |x| given the sign s of x: fabs for plain scalars (bit-exact), s * x on duals (the derivative).
-__device__ __forceinline__ float absSigned(float x, float) { return fabsf(x); }
-__device__ __forceinline__ double absSigned(double x, double) { return fabs(x); }
-template <class T, int K> __device__ __forceinline__ Dual<T, K> absSigned(const Dual<T, K> &x, const Dual<T, K> &s)
+template <class T>
+__device__ __forceinline__ bool edgeProject(const V3<T> &a, const V3<T> &b, T wA, T wB, T rest, T compliance, T lambda, T dt,
+                                            T relax, V3<T> &cA, V3<T> &cB, T &lambdaOut)
 {
-    return s * x;
+    EdgeTerms<T> e;
+    lambdaOut = lambda;
+    if (!edgeTerms(a, b, wA, wB, rest, compliance, lambda, dt, e)) return false;
+    const V3<T> gA = (-e.delta) / e.len;
+    const V3<T> gB = -gA;
+    lambdaOut = lambda + e.dl;
+    cA = ((wA * e.dl) * gA) * relax;
+    cB = ((wB * e.dl) * gB) * relax;
+    return true;
 }
 
-// physics_soft_solve_tet_constraints.cs.hlsl:15-87 (k_solveTets).  Returns false when the
-// reference keeps the previous record (no mass, no denominator).
-template <class S, class T>
-__device__ __forceinline__ bool tetProject(const V3<S> p[4], const T w[4], T rest, const S &compliance,
-                                           const S &lambda, T dt, T relax, V3<S> out[4], S &lambdaOut)
+// Adjoints of b (that of a is its negative) and lambda from those of the corrections and of lambda'.
+// With u = delta / len: cA = -wA relax dl u, cB = wB relax dl u.
+template <class T>
+__device__ __forceinline__ V3<T> edgeAdjoint(const EdgeTerms<T> &e, T wA, T wB, T relax, const V3<T> &gA, const V3<T> &gB, T gL,
+                                             T &gLambda)
+{
+    const V3<T> u = e.delta / e.len;
+    const V3<T> m = (gB * (wB * relax)) - (gA * (wA * relax));
+    const T D = gL + dot3(m, u);          // of dl
+    const V3<T> U = m * e.dl;             // of u
+    gLambda = gL - D * (e.alpha / e.den);
+    return (u * (-D / e.den)) + ((U - (u * dot3(U, u))) / e.len);
+}
+
+// physics_soft_solve_tet_constraints.cs.hlsl:15-87 (k_solveTets).  False when the reference keeps the
+// previous record (no mass, no denominator).
+template <class T> struct TetTerms {
+    V3<T> e1, e2, e3; // p1 - p0, p2 - p0, p3 - p0
+    V3<T> a, b;       // p3 - p1, p2 - p1
+    V3<T> g[4];
+    T k6, alpha, den, dl;
+};
+template <class T>
+__device__ __forceinline__ bool tetTerms(const V3<T> p[4], const T w[4], T rest, T compliance, T lambda, T dt, TetTerms<T> &t)
 {
     const T eps = T(1.0e-6);
-    lambdaOut = lambda;
     if ((w[0] + w[1] + w[2] + w[3]) <= eps) return false;
-    const S sv = dot3(cross3(p[1] - p[0], p[2] - p[0]), p[3] - p[0]) / cst(lambda, 6.0);
-    const T vsv = val(sv) >= T(0) ? T(1) : T(-1);
-    const S vs = cst(lambda, vsv);
-    const S Cv = absSigned(sv, vs) - cst(lambda, rest > T(0) ? rest : T(0));
-    const S k6 = vs / cst(lambda, 6.0);
-    const V3<S> g0 = cross3(p[3] - p[1], p[2] - p[1]) * k6;
-    const V3<S> g1 = cross3(p[2] - p[0], p[3] - p[0]) * k6;
-    const V3<S> g2 = cross3(p[3] - p[0], p[1] - p[0]) * k6;
-    const V3<S> g3 = cross3(p[1] - p[0], p[2] - p[0]) * k6;
-    const S sg = cst(lambda, w[0]) * dot3(g0, g0) + cst(lambda, w[1]) * dot3(g1, g1) +
-                 cst(lambda, w[2]) * dot3(g2, g2) + cst(lambda, w[3]) * dot3(g3, g3);
+    t.e1 = p[1] - p[0];
+    t.e2 = p[2] - p[0];
+    t.e3 = p[3] - p[0];
+    t.a = p[3] - p[1];
+    t.b = p[2] - p[1];
+    const T sv = dot3(cross3(t.e1, t.e2), t.e3) / T(6);
+    const T vs = sv >= T(0) ? T(1) : T(-1);
+    const T Cv = absD(sv) - (rest > T(0) ? rest : T(0));
+    t.k6 = vs / T(6);
+    t.g[0] = cross3(t.a, t.b) * t.k6;
+    t.g[1] = cross3(t.e2, t.e3) * t.k6;
+    t.g[2] = cross3(t.e3, t.e1) * t.k6;
+    t.g[3] = cross3(t.e1, t.e2) * t.k6;
+    const T sg = w[0] * dot3(t.g[0], t.g[0]) + w[1] * dot3(t.g[1], t.g[1]) + w[2] * dot3(t.g[2], t.g[2]) +
+                 w[3] * dot3(t.g[3], t.g[3]);
     const T dt2 = dt * dt;
-    const S alpha = compliance / cst(lambda, dt2 > eps ? dt2 : eps);
-    const S den = sg + alpha;
-    if (!(val(den) > eps)) return false;
-    const S dl = -(Cv + alpha * lambda) / den;
-    lambdaOut = lambda + dl;
-    const V3<S> g[4] = {g0, g1, g2, g3};
-#pragma unroll
-    for (int k = 0; k < 4; ++k) out[k] = ((cst(lambda, w[k]) * dl) * g[k]) * cst(lambda, relax);
+    t.alpha = compliance / (dt2 > eps ? dt2 : eps);
+    t.den = sg + t.alpha;
+    if (!(t.den > eps)) return false;
+    t.dl = -(Cv + t.alpha * lambda) / t.den;
     return true;
 }
 
+// Adjoints of the four positions, lambda and the scaled compliance from those of the corrections (gC) and
+// of lambda'.  With out_j = w_j relax dl g_j and dl = -(C + alpha lambda) / den, den = sum w_j |g_j|^2 + alpha;
+// the gradients are cross products, whose adjoints are cross products, and dC / dp_j = g_j.
+template <class T>
+__device__ __forceinline__ void tetAdjoint(const TetTerms<T> &t, const T w[4], T relax, const V3<T> gC[4], T lambda, T gL,
+                                           V3<T> gP[4], T &gLambda, T &gAlpha)
+{
+    T D = gL;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) D += (w[j] * relax) * dot3(gC[j], t.g[j]);
+    const T inv = T(1) / t.den;
+    const T S = -(D * t.dl) * inv; // of den
+    const T V = -D * inv;          // of C
+    gLambda = gL + V * t.alpha;
+    gAlpha = V * lambda + S;
+    V3<T> h[4];                    // of k6 x the cross products
+#pragma unroll
+    for (int j = 0; j < 4; ++j) h[j] = ((gC[j] * (w[j] * relax * t.dl)) + (t.g[j] * (T(2) * w[j] * S))) * t.k6;
+    const V3<T> gE1 = cross3(h[2], t.e3) + cross3(t.e2, h[3]);
+    const V3<T> gE2 = cross3(t.e3, h[1]) + cross3(h[3], t.e1);
+    const V3<T> gE3 = cross3(h[1], t.e2) + cross3(t.e1, h[2]);
+    const V3<T> ga = cross3(t.b, h[0]), gb = cross3(h[0], t.a);
+    gP[0] = (t.g[0] * V) - (gE1 + gE2 + gE3);
+    gP[1] = (t.g[1] * V) + (gE1 - (ga + gb));
+    gP[2] = (t.g[2] * V) + (gE2 + gb);
+    gP[3] = (t.g[3] * V) + (gE3 + ga);
+}
 
 // ---------------------------------------------------------------- device scene
 template <class T> struct DScene {
@@ -205,15 +189,24 @@ template <class T> struct DScene {
     const uint32_t *edgeEnabled = nullptr;
     const uint4 *tetIdx = nullptr;
     const T *tetRest = nullptr;
-    const uint2 *edgeRanges = nullptr, *edgeInc = nullptr, *tetRanges = nullptr, *tetInc = nullptr;
+    // per particle its records (first, count), per constraint entry the record it writes (kNone: none)
+    const uint2 *edgeRanges = nullptr, *tetRanges = nullptr;
+    const uint2 *edgeDst = nullptr;
+    const uint4 *tetDst = nullptr;
     T g[3] = {T(0), T(0), T(0)};
     T relax = T(0.2);
 };
 
 template <class T> __device__ __forceinline__ V3<T> xyzOf(const P4<T> &p) { return {p.x, p.y, p.z}; }
 
-// k_predictKeys for a solid particle (gravity scale 1)
-template <class T> __global__ void k_dPredict(DScene<T> s, P4<T> *x, P4<T> *v, P4<T> *xprev, T dt)
+constexpr uint32_t kNone = 0xffffffffu;
+template <class T> __device__ __forceinline__ void putRecord(P4<T> *records, uint32_t at, const V3<T> &v)
+{
+    if (at != kNone) records[at] = {v.x, v.y, v.z, T(0)};
+}
+
+// k_predictKeys for a solid particle (gravity scale 1): the predicted positions go to xOut
+template <class T> __global__ void k_dPredict(DScene<T> s, const P4<T> *x, P4<T> *xOut, P4<T> *v, P4<T> *xprev, T dt)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= s.N) return;
@@ -221,6 +214,7 @@ template <class T> __global__ void k_dPredict(DScene<T> s, P4<T> *x, P4<T> *v, P
     xprev[i] = {p.x, p.y, p.z, T(0)};
     if (s.w[i] <= T(1.0e-6)) {
         v[i] = {T(0), T(0), T(0), T(0)};
+        xOut[i] = p;
         return;
     }
     const P4<T> vv = v[i];
@@ -228,66 +222,106 @@ template <class T> __global__ void k_dPredict(DScene<T> s, P4<T> *x, P4<T> *v, P
     const V3<T> vel = V3<T>{vv.x, vv.y, vv.z} + V3<T>{s.g[0], s.g[1], s.g[2]} * gs;
     const V3<T> pp = V3<T>{p.x, p.y, p.z} + vel * dt;
     v[i] = {vel.x, vel.y, vel.z, T(0)};
-    x[i] = {pp.x, pp.y, pp.z, p.w};
+    xOut[i] = {pp.x, pp.y, pp.z, p.w};
 }
 
+// The iteration kernels are launched with programmatic stream serialization: what their predecessor does
+// not write loads ahead of the wait (as in the solver's kernels: cn::pdlEnter).
 template <class T>
-__global__ void k_dEdges(DScene<T> s, const P4<T> *x, T *lambda, P4<T> *corr, T dt)
+__global__ void __launch_bounds__(kDiffThreads) k_dEdges(DScene<T> s, const P4<T> *x, const T *lambdaIn, T *lambdaOut, P4<T> *corr,
+                                                         T dt, bool first)
 {
     const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
+    uint2 ab = make_uint2(0u, 0u), d = make_uint2(kNone, kNone);
+    T wA = T(0), wB = T(0), rest = T(0), comp = T(0), lambda = T(0);
+    bool enabled = false;
+    if (e < s.E) {
+        ab = s.edgePair[e];
+        d = s.edgeDst[e];
+        wA = s.w[ab.x];
+        wB = s.w[ab.y];
+        rest = s.edgeRest[e];
+        comp = s.edgeCompliance[e] > T(0) ? s.edgeCompliance[e] : T(0);
+        if (!first) lambda = lambdaIn[e];
+        enabled = s.edgeEnabled[e] != 0u;
+    }
+    cn::pdlEnter();
     if (e >= s.E) return;
-    const uint2 ab = s.edgePair[e];
     V3<T> cA{T(0), T(0), T(0)}, cB = cA;
-    T lo = lambda[e];
-    if (s.edgeEnabled[e] != 0u)
-        edgeProject<T, T>(xyzOf(x[ab.x]), xyzOf(x[ab.y]), s.w[ab.x], s.w[ab.y], s.edgeRest[e],
-                          s.edgeCompliance[e] > T(0) ? s.edgeCompliance[e] : T(0), lambda[e], dt, s.relax, cA, cB, lo);
-    lambda[e] = lo;
-    corr[2 * e] = {cA.x, cA.y, cA.z, T(0)};
-    corr[2 * e + 1] = {cB.x, cB.y, cB.z, T(0)};
+    T lo = lambda;
+    if (enabled) edgeProject<T>(xyzOf(x[ab.x]), xyzOf(x[ab.y]), wA, wB, rest, comp, lambda, dt, s.relax, cA, cB, lo);
+    lambdaOut[e] = lo;
+    putRecord(corr, d.x, cA);
+    putRecord(corr, d.y, cB);
 }
 
 template <class T>
-__global__ void k_dTets(DScene<T> s, const P4<T> *x, const T *compliance, T *lambda, P4<T> *corr, T dt)
+__global__ void __launch_bounds__(kDiffThreads) k_dTets(DScene<T> s, const P4<T> *x, const T *compliance, const T *lambdaIn,
+                                                        T *lambdaOut, P4<T> *corr, T dt, bool first)
 {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= s.T_) return;
-    const uint4 q = s.tetIdx[t];
-    const uint32_t id[4] = {q.x, q.y, q.z, q.w};
-    V3<T> p[4];
-    T w[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        p[k] = xyzOf(x[id[k]]);
-        w[k] = s.w[id[k]];
+    uint4 q = make_uint4(0u, 0u, 0u, 0u), d = make_uint4(kNone, kNone, kNone, kNone);
+    T w[4] = {T(0), T(0), T(0), T(0)}, rest = T(0), comp = T(0), lambda = T(0);
+    if (t < s.T_) {
+        q = s.tetIdx[t];
+        d = s.tetDst[t];
+        w[0] = s.w[q.x];
+        w[1] = s.w[q.y];
+        w[2] = s.w[q.z];
+        w[3] = s.w[q.w];
+        rest = s.tetRest[t];
+        comp = compliance[t] > T(0) ? compliance[t] : T(0);
+        if (!first) lambda = lambdaIn[t];
     }
-    V3<T> out[4];
-    T lo;
-    if (!tetProject<T, T>(p, w, s.tetRest[t], compliance[t] > T(0) ? compliance[t] : T(0), lambda[t], dt, s.relax,
-                          out, lo))
-        return; // the previous record stays (the reference's behaviour)
-    lambda[t] = lo;
+    cn::pdlEnter();
+    if (t >= s.T_) return;
+    const V3<T> p[4] = {xyzOf(x[q.x]), xyzOf(x[q.y]), xyzOf(x[q.z]), xyzOf(x[q.w])};
+    TetTerms<T> m;
+    if (!tetTerms<T>(p, w, rest, comp, lambda, dt, m)) { // the previous record stays (the reference's behaviour)
+        lambdaOut[t] = lambda;
+        return;
+    }
+    lambdaOut[t] = lambda + m.dl;
+    const uint32_t dst[4] = {d.x, d.y, d.z, d.w};
 #pragma unroll
-    for (int k = 0; k < 4; ++k) corr[4 * t + k] = {out[k].x, out[k].y, out[k].z, T(0)};
+    for (int k = 0; k < 4; ++k) putRecord(corr, dst[k], ((w[k] * m.dl) * m.g[k]) * s.relax);
 }
 
-// k_applyPair / k_applyQuad
-template <class T, int kPer>
-__global__ void k_dApply(DScene<T> s, P4<T> *x, const uint2 *ranges, const uint2 *inc, const P4<T> *corr)
+// out[i] = in[i] + the sum of i's records in ascending constraint order: the apply of a family (k_applyGather;
+// particles without mass keep their position), and of the adjoint records (kAdjoint: every particle).
+// Four lanes per particle, one per component, sixteen records in flight.  In place when out == in.
+constexpr uint32_t kLanes = 4u, kAhead = 16u;
+template <class T, bool kAdjoint>
+__global__ void __launch_bounds__(kDiffThreads) k_dGather(DScene<T> s, const P4<T> *in, P4<T> *out, const uint2 *ranges,
+                                                          const P4<T> *records)
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= s.N) return;
-    if (s.w[i] <= T(1.0e-6)) return;
-    const P4<T> p = x[i];
-    const uint2 r = ranges[i];
-    V3<T> total{T(0), T(0), T(0)};
-    for (uint32_t k = 0; k < r.y; ++k) {
-        const uint2 ref = inc[r.x + k];
-        const P4<T> c = corr[kPer * ref.x + (kPer == 2 ? (ref.y == 0u ? 0u : 1u) : (ref.y > 3u ? 3u : ref.y))];
-        total = total + V3<T>{c.x, c.y, c.z};
+    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x, i = q / kLanes, comp = q % kLanes;
+    const bool live = i < s.N;
+    T x = T(0);
+    bool moves = false;
+    uint2 r = make_uint2(0u, 0u);
+    if (live) {
+        x = reinterpret_cast<const T *>(in)[q]; // not written by the solve this kernel follows
+        r = ranges[i];
+        moves = comp < 3u && (kAdjoint || s.w[i] > T(1.0e-6));
     }
-    const V3<T> n = V3<T>{p.x, p.y, p.z} + total;
-    x[i] = {n.x, n.y, n.z, p.w};
+    cn::pdlEnter();
+    if (!live) return;
+    if (moves) {
+        const T *src = reinterpret_cast<const T *>(records + r.x) + comp;
+        T total = kAdjoint ? x : T(0);
+        for (uint32_t k = 0; k < r.y; k += kAhead) {
+            T c[kAhead];
+#pragma unroll
+            for (uint32_t j = 0; j < kAhead; ++j)
+                if (k + j < r.y) c[j] = src[kLanes * (k + j)];
+#pragma unroll
+            for (uint32_t j = 0; j < kAhead; ++j)
+                if (k + j < r.y) total += c[j];
+        }
+        x = kAdjoint ? total : x + total;
+    }
+    if (moves || out != in) reinterpret_cast<T *>(out)[q] = kAdjoint && comp == 3u ? T(0) : x;
 }
 
 // k_updateVelocities for a solid particle
@@ -307,111 +341,85 @@ template <class T> __global__ void k_dVelocity(DScene<T> s, const P4<T> *x, cons
 }
 
 // ---------------------------------------------------------------- adjoint kernels
-// Edge: inputs (a xyz, b xyz, lambda, compliance) -> outputs (cA, cB, lambda').  Writes the
-// adjoints of a and b as records (2 per edge), accumulates d loss / d lambda into gLambda
-// (replaced by the adjoint of the input lambda).  Edge compliance is not a parameter here.
+// Edge: the adjoints of a and b as records, that of the input lambda in gLambda's place.  Edge
+// compliance is not a parameter here.  Corrections reach particles with mass only (the apply skips
+// the rest), so the others' adjoints do not enter.
 template <class T>
-__global__ void k_dEdgesBack(DScene<T> s, const P4<T> *x, const T *lambdaIn, const P4<T> *gX, T *gLambda,
-                             P4<T> *rec, T dt)
+__global__ void __launch_bounds__(kDiffThreads) k_dEdgesBack(DScene<T> s, const P4<T> *x, const T *lambdaIn, const P4<T> *gX,
+                                                             T *gLambda, P4<T> *rec, T dt)
 {
     const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= s.E) return;
-    const uint2 ab = s.edgePair[e];
-    typedef Dual<T, 7> D;
-    V3<D> a, b;
-    const V3<T> xa = xyzOf(x[ab.x]), xb = xyzOf(x[ab.y]);
-    a = {mkc<T, 7>(xa.x), mkc<T, 7>(xa.y), mkc<T, 7>(xa.z)};
-    b = {mkc<T, 7>(xb.x), mkc<T, 7>(xb.y), mkc<T, 7>(xb.z)};
-    a.x.d[0] = a.y.d[1] = a.z.d[2] = T(1);
-    b.x.d[3] = b.y.d[4] = b.z.d[5] = T(1);
-    D lam = mkc<T, 7>(lambdaIn[e]);
-    lam.d[6] = T(1);
-    const D comp = mkc<T, 7>(s.edgeCompliance[e] > T(0) ? s.edgeCompliance[e] : T(0));
-    V3<D> cA{mkc<T, 7>(T(0)), mkc<T, 7>(T(0)), mkc<T, 7>(T(0))}, cB = cA;
-    D lo = lam;
+    uint2 ab = make_uint2(0u, 0u), d = make_uint2(kNone, kNone);
+    T wA = T(0), wB = T(0), gl = T(0), lambda = T(0);
+    V3<T> a{T(0), T(0), T(0)}, b = a;
+    EdgeTerms<T> m{};
     bool wrote = false;
-    if (s.edgeEnabled[e] != 0u)
-        wrote = edgeProject<D, T>(a, b, s.w[ab.x], s.w[ab.y], s.edgeRest[e], comp, lam, dt, s.relax, cA, cB, lo);
-    // upstream adjoints: corrections reach particles with mass only (the apply skips the rest)
-    const T gl = gLambda[e];
-    T gin[7];
-#pragma unroll
-    for (int k = 0; k < 7; ++k) gin[k] = gl * lo.d[k];
-    if (wrote) {
-        const P4<T> ga = s.w[ab.x] > T(1.0e-6) ? gX[ab.x] : P4<T>{T(0), T(0), T(0), T(0)};
-        const P4<T> gb = s.w[ab.y] > T(1.0e-6) ? gX[ab.y] : P4<T>{T(0), T(0), T(0), T(0)};
-#pragma unroll
-        for (int k = 0; k < 7; ++k)
-            gin[k] += ga.x * cA.x.d[k] + ga.y * cA.y.d[k] + ga.z * cA.z.d[k] + gb.x * cB.x.d[k] + gb.y * cB.y.d[k] +
-                      gb.z * cB.z.d[k];
+    if (e < s.E) { // the forward's state: recorded before the adjoint began
+        ab = s.edgePair[e];
+        d = s.edgeDst[e];
+        wA = s.w[ab.x];
+        wB = s.w[ab.y];
+        gl = gLambda[e];
+        lambda = lambdaIn[e];
+        a = xyzOf(x[ab.x]);
+        b = xyzOf(x[ab.y]);
+        const T comp = s.edgeCompliance[e] > T(0) ? s.edgeCompliance[e] : T(0);
+        wrote = s.edgeEnabled[e] != 0u && edgeTerms<T>(a, b, wA, wB, s.edgeRest[e], comp, lambda, dt, m);
     }
-    rec[2 * e] = {gin[0], gin[1], gin[2], T(0)};
-    rec[2 * e + 1] = {gin[3], gin[4], gin[5], T(0)};
-    gLambda[e] = gin[6];
+    cn::pdlEnter();
+    if (e >= s.E) return;
+    V3<T> gB{T(0), T(0), T(0)};
+    if (wrote) {
+        const V3<T> zero{T(0), T(0), T(0)};
+        gB = edgeAdjoint<T>(m, wA, wB, s.relax, wA > T(1.0e-6) ? xyzOf(gX[ab.x]) : zero,
+                            wB > T(1.0e-6) ? xyzOf(gX[ab.y]) : zero, gl, gl);
+    }
+    putRecord(rec, d.x, -gB);
+    putRecord(rec, d.y, gB);
+    gLambda[e] = gl;
 }
 
-// Tet: inputs (4 positions, lambda, compliance) -> outputs (4 corrections, lambda').
+// Tet: the adjoints of the four positions as records, of lambda in place, of the compliance added up.
 template <class T>
-__global__ void k_dTetsBack(DScene<T> s, const P4<T> *x, const T *compliance, const T *lambdaIn, const P4<T> *gX,
-                            T *gLambda, P4<T> *rec, T *gCompliance, T dt)
+__global__ void __launch_bounds__(kDiffThreads) k_dTetsBack(DScene<T> s, const P4<T> *x, const T *compliance, const T *lambdaIn,
+                                                            const P4<T> *gX, T *gLambda, P4<T> *rec, T *gCompliance, T dt)
 {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    uint4 q = make_uint4(0u, 0u, 0u, 0u), d = make_uint4(kNone, kNone, kNone, kNone);
+    T w[4] = {T(0), T(0), T(0), T(0)}, lambda = T(0), gl = T(0), c0 = T(0);
+    TetTerms<T> m{};
+    bool wrote = false;
+    if (t < s.T_) {
+        q = s.tetIdx[t];
+        d = s.tetDst[t];
+        w[0] = s.w[q.x];
+        w[1] = s.w[q.y];
+        w[2] = s.w[q.z];
+        w[3] = s.w[q.w];
+        lambda = lambdaIn[t];
+        gl = gLambda[t];
+        c0 = compliance[t];
+        const V3<T> p[4] = {xyzOf(x[q.x]), xyzOf(x[q.y]), xyzOf(x[q.z]), xyzOf(x[q.w])};
+        wrote = tetTerms<T>(p, w, s.tetRest[t], c0 > T(0) ? c0 : T(0), lambda, dt, m);
+    }
+    cn::pdlEnter();
     if (t >= s.T_) return;
-    typedef Dual<T, 14> D;
-    const uint4 q = s.tetIdx[t];
-    const uint32_t id[4] = {q.x, q.y, q.z, q.w};
-    V3<D> p[4];
-    T w[4];
+    const uint32_t id[4] = {q.x, q.y, q.z, q.w}, dst[4] = {d.x, d.y, d.z, d.w};
+    V3<T> gP[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const V3<T> xp = xyzOf(x[id[k]]);
-        p[k] = {mkc<T, 14>(xp.x), mkc<T, 14>(xp.y), mkc<T, 14>(xp.z)};
-        p[k].x.d[3 * k] = p[k].y.d[3 * k + 1] = p[k].z.d[3 * k + 2] = T(1);
-        w[k] = s.w[id[k]];
-    }
-    D lam = mkc<T, 14>(lambdaIn[t]);
-    lam.d[12] = T(1);
-    const T c0 = compliance[t];
-    D comp = mkc<T, 14>(c0 > T(0) ? c0 : T(0));
-    comp.d[13] = c0 > T(0) ? T(1) : T(0);
-    V3<D> out[4];
-    D lo;
-    const bool wrote = tetProject<D, T>(p, w, s.tetRest[t], comp, lam, dt, s.relax, out, lo);
-    const T gl = gLambda[t];
-    T gin[14];
-#pragma unroll
-    for (int k = 0; k < 14; ++k) gin[k] = wrote ? gl * lo.d[k] : (k == 12 ? gl : T(0));
+    for (int j = 0; j < 4; ++j) gP[j] = {T(0), T(0), T(0)};
     if (wrote) {
+        V3<T> gC[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            if (w[j] <= T(1.0e-6)) continue;
-            const P4<T> g = gX[id[j]];
-#pragma unroll
-            for (int k = 0; k < 14; ++k) gin[k] += g.x * out[j].x.d[k] + g.y * out[j].y.d[k] + g.z * out[j].z.d[k];
-        }
+        for (int j = 0; j < 4; ++j) gC[j] = w[j] > T(1.0e-6) ? xyzOf(gX[id[j]]) : V3<T>{T(0), T(0), T(0)};
+        T gAlpha;
+        tetAdjoint<T>(m, w, s.relax, gC, lambda, gl, gP, gl, gAlpha);
+        const T dt2 = dt * dt;
+        if (c0 > T(0)) gCompliance[t] += gAlpha / (dt2 > T(1.0e-6) ? dt2 : T(1.0e-6));
     }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) rec[4 * t + j] = {gin[3 * j], gin[3 * j + 1], gin[3 * j + 2], T(0)};
-    gLambda[t] = gin[12];
-    gCompliance[t] += gin[13];
-}
-
-// gX_in[i] = gX_out[i] + sum of the records of i's incident constraints (ascending order)
-template <class T, int kPer>
-__global__ void k_dGather(DScene<T> s, const P4<T> *gOut, P4<T> *gIn, const uint2 *ranges, const uint2 *inc,
-                          const P4<T> *rec)
-{
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= s.N) return;
-    const P4<T> g = gOut[i];
-    const uint2 r = ranges[i];
-    V3<T> total{g.x, g.y, g.z};
-    for (uint32_t k = 0; k < r.y; ++k) {
-        const uint2 ref = inc[r.x + k];
-        const P4<T> c = rec[kPer * ref.x + (kPer == 2 ? (ref.y == 0u ? 0u : 1u) : (ref.y > 3u ? 3u : ref.y))];
-        total = total + V3<T>{c.x, c.y, c.z};
-    }
-    gIn[i] = {total.x, total.y, total.z, T(0)};
+    for (int j = 0; j < 4; ++j) putRecord(rec, dst[j], gP[j]);
+    gLambda[t] = gl;
 }
 
 // Velocity update + predict, backwards.  In: gX (adjoint of the substep's end positions),
@@ -475,8 +483,10 @@ template <class T> struct Engine {
     P4<T> *gX = nullptr, *gV = nullptr, *gA = nullptr, *gB = nullptr;
     T *gLE = nullptr, *gLT = nullptr;
     P4<T> *recE = nullptr, *recT = nullptr;
-    const T *compliance = nullptr;            // the forward's tet compliances (caller's device buffer)
+    T *compliance = nullptr, *gCompliance = nullptr; // the forward's tet compliances, their adjoint
     bool forwardDone = false;
+    // one substep, and one substep with its iteration states and its adjoint, on the buffers above
+    cudaGraphExec_t stepGraph = nullptr, adjointGraph = nullptr;
 
     template <class U> U *alloc(size_t n)
     {
@@ -490,6 +500,9 @@ template <class T> struct Engine {
     }
     void release()
     {
+        if (stepGraph) cudaGraphExecDestroy(stepGraph);
+        if (adjointGraph) cudaGraphExecDestroy(adjointGraph);
+        stepGraph = adjointGraph = nullptr;
         for (void *p : owned)
             if (p) cudaFree(p);
         owned.clear();
@@ -501,53 +514,125 @@ void copyAsync(void *dst, const void *src, size_t bytes, cudaStream_t st)
     if (bytes) cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, st);
 }
 
-template <class T> void runIteration(Engine<T> &g, P4<T> *x, cudaStream_t st)
+template <class... P, class... A> void launchDependent(void (*k)(P...), size_t threads, cudaStream_t st, A... args)
 {
-    const DScene<T> &s = g.s;
-    if (s.E) {
-        k_dEdges<T><<<gridOf(s.E), kDiffThreads, 0, st>>>(s, x, g.lamE, g.corrE, g.dt);
-        k_dApply<T, 2><<<gridOf(s.N), kDiffThreads, 0, st>>>(s, x, s.edgeRanges, s.edgeInc, g.corrE);
-    }
-    if (s.T_) {
-        k_dTets<T><<<gridOf(s.T_), kDiffThreads, 0, st>>>(s, x, g.compliance, g.lamT, g.corrT, g.dt);
-        k_dApply<T, 4><<<gridOf(s.N), kDiffThreads, 0, st>>>(s, x, s.tetRanges, s.tetInc, g.corrT);
-    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(gridOf(threads), 1, 1);
+    cfg.blockDim = dim3(kDiffThreads, 1, 1);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k, P(args)...);
 }
 
-// One substep from (x, v) in place; with `record`, the iteration states for the adjoint.
-template <class T> void runSubstep(Engine<T> &g, P4<T> *x, P4<T> *v, bool record, cudaStream_t st)
+// One substep of the state (g.x, g.v).  With `record` every iteration writes its positions and lambdas to
+// the next slot of the iteration states instead of in place, for the adjoint: edges of iteration `it` at
+// (itX0, itLE)[it], tets at (itX1, itLT)[it].
+template <class T> void runSubstep(Engine<T> &g, bool record, cudaStream_t st)
 {
     const DScene<T> &s = g.s;
-    const size_t nb = sizeof(P4<T>) * s.N;
-    k_dPredict<T><<<gridOf(s.N), kDiffThreads, 0, st>>>(s, x, v, g.xprev, g.dt);
-    if (s.E) cudaMemsetAsync(g.lamE, 0, sizeof(T) * s.E, st);
-    if (s.T_) cudaMemsetAsync(g.lamT, 0, sizeof(T) * s.T_, st);
+    const size_t lanes = size_t(s.N) * kLanes;
+    P4<T> *cur = record ? g.itX0 : g.x;
+    k_dPredict<T><<<gridOf(s.N), kDiffThreads, 0, st>>>(s, g.x, cur, g.v, g.xprev, g.dt);
     for (uint32_t it = 0; it < g.iterations; ++it) {
-        if (record) {
-            copyAsync(g.itX0 + size_t(it) * s.N, x, nb, st);
-            copyAsync(g.itLE + size_t(it) * s.E, g.lamE, sizeof(T) * s.E, st);
-        }
+        const bool last = it + 1u == g.iterations, first = it == 0u;
+        P4<T> *done = !record ? g.x : last ? g.x : g.itX0 + size_t(it + 1u) * s.N;
         if (s.E) {
-            k_dEdges<T><<<gridOf(s.E), kDiffThreads, 0, st>>>(s, x, g.lamE, g.corrE, g.dt);
-            k_dApply<T, 2><<<gridOf(s.N), kDiffThreads, 0, st>>>(s, x, s.edgeRanges, s.edgeInc, g.corrE);
-        }
-        if (record) {
-            copyAsync(g.itX1 + size_t(it) * s.N, x, nb, st);
-            copyAsync(g.itLT + size_t(it) * s.T_, g.lamT, sizeof(T) * s.T_, st);
+            T *in = record ? g.itLE + size_t(it) * s.E : g.lamE;
+            T *out = record && !last ? in + s.E : g.lamE;
+            P4<T> *to = record && s.T_ ? g.itX1 + size_t(it) * s.N : done;
+            launchDependent(k_dEdges<T>, s.E, st, s, cur, in, out, g.corrE, g.dt, first);
+            launchDependent(k_dGather<T, false>, lanes, st, s, cur, to, s.edgeRanges, g.corrE);
+            cur = to;
         }
         if (s.T_) {
-            k_dTets<T><<<gridOf(s.T_), kDiffThreads, 0, st>>>(s, x, g.compliance, g.lamT, g.corrT, g.dt);
-            k_dApply<T, 4><<<gridOf(s.N), kDiffThreads, 0, st>>>(s, x, s.tetRanges, s.tetInc, g.corrT);
+            T *in = record ? g.itLT + size_t(it) * s.T_ : g.lamT;
+            T *out = record && !last ? in + s.T_ : g.lamT;
+            launchDependent(k_dTets<T>, s.T_, st, s, cur, g.compliance, in, out, g.corrT, g.dt, first);
+            launchDependent(k_dGather<T, false>, lanes, st, s, cur, done, s.tetRanges, g.corrT);
+            cur = done;
         }
     }
-    k_dVelocity<T><<<gridOf(s.N), kDiffThreads, 0, st>>>(s, x, g.xprev, v, g.dt);
+    if (cur != g.x) copyAsync(g.x, cur, sizeof(P4<T>) * s.N, st); // neither edges nor tets
+    k_dVelocity<T><<<gridOf(s.N), kDiffThreads, 0, st>>>(s, g.x, g.xprev, g.v, g.dt);
+}
+
+// The substep from (g.x, g.v) with its iteration states, then its adjoint: (g.gX, g.gV) from those of its end
+// to those of its start, the compliances' added to g.gCompliance.
+template <class T> void runAdjoint(Engine<T> &g, cudaStream_t st)
+{
+    const DScene<T> &s = g.s;
+    const size_t lanes = size_t(s.N) * kLanes;
+    runSubstep(g, true, st);
+    P4<T> *gA = g.gA, *gB = g.gB; // gA: the adjoint entering the last iteration's output
+    k_dVelocityBack<T><<<gridOf(s.N), kDiffThreads, 0, st>>>(s, g.gX, g.gV, gA, g.dt);
+    if (s.E) cudaMemsetAsync(g.gLE, 0, sizeof(T) * s.E, st);
+    if (s.T_) cudaMemsetAsync(g.gLT, 0, sizeof(T) * s.T_, st);
+    for (int it = int(g.iterations) - 1; it >= 0; --it) {
+        if (s.T_) {
+            const P4<T> *x = (s.E ? g.itX1 : g.itX0) + size_t(it) * s.N;
+            launchDependent(k_dTetsBack<T>, s.T_, st, s, x, g.compliance, g.itLT + size_t(it) * s.T_, gA, g.gLT, g.recT,
+                            g.gCompliance, g.dt);
+            launchDependent(k_dGather<T, true>, lanes, st, s, gA, gB, s.tetRanges, g.recT);
+            std::swap(gA, gB);
+        }
+        if (s.E) {
+            launchDependent(k_dEdgesBack<T>, s.E, st, s, g.itX0 + size_t(it) * s.N, g.itLE + size_t(it) * s.E, gA, g.gLE,
+                            g.recE, g.dt);
+            launchDependent(k_dGather<T, true>, lanes, st, s, gA, gB, s.edgeRanges, g.recE);
+            std::swap(gA, gB);
+        }
+    }
+    // predict backwards: (gX, gV) of the substep start
+    k_dPredictBack<T><<<gridOf(s.N), kDiffThreads, 0, st>>>(s, gA, g.gV, g.gX, g.gV, g.dt);
+}
+
+// Runs one of the two through its graph, captured at first use; on a stream that is itself being captured
+// (a caller's graph) the launches go there one by one.
+template <class T, class F> cn_status replay(Engine<T> &g, cudaGraphExec_t &exec, cudaStream_t own, cudaStream_t st, F &&enqueue)
+{
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess) {
+        cudaGetLastError(); // the legacy stream beside somebody's capture: not this stream's
+        capturing = cudaStreamCaptureStatusNone;
+    }
+    if (capturing != cudaStreamCaptureStatusNone) {
+        enqueue(g, st);
+        return CN_OK;
+    }
+    if (!exec) {
+        cudaGraph_t graph = nullptr;
+        cudaError_t e = cudaStreamBeginCapture(own, cudaStreamCaptureModeThreadLocal);
+        if (e == cudaSuccess) {
+            enqueue(g, own);
+            e = cudaStreamEndCapture(own, &graph);
+        }
+        if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
+        if (graph) cudaGraphDestroy(graph);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            exec = nullptr;
+            return setError(CN_ERR_CUDA, std::string("cn_diff: graph capture failed: ") + cudaGetErrorString(e));
+        }
+    }
+    const cudaError_t e = cudaGraphLaunch(exec, st);
+    if (e != cudaSuccess) return setError(CN_ERR_CUDA, std::string("cn_diff: ") + cudaGetErrorString(e));
+    return CN_OK;
+}
+
+template <class T> cn_status step(Engine<T> &g, cudaStream_t own, cudaStream_t st)
+{
+    return replay(g, g.stepGraph, own, st, [](Engine<T> &e, cudaStream_t on) { runSubstep(e, false, on); });
 }
 
 template <class T> cn_status forward(Engine<T> &g, const T *compliance, const P4<T> *x0, const P4<T> *v0, P4<T> *xOut,
-                                     P4<T> *vOut, cudaStream_t st)
+                                     P4<T> *vOut, cudaStream_t own, cudaStream_t st)
 {
     const size_t nb = sizeof(P4<T>) * g.s.N;
-    g.compliance = compliance;
+    if (g.s.T_) cudaMemcpyAsync(g.compliance, compliance, sizeof(T) * g.s.T_, cudaMemcpyDefault, st);
     copyAsync(g.x, x0, nb, st);
     copyAsync(g.v, v0, nb, st);
     // corrections start at zero (the solver's upload clears them)
@@ -559,7 +644,8 @@ template <class T> cn_status forward(Engine<T> &g, const T *compliance, const P4
             copyAsync(g.ckX + c * g.s.N, g.x, nb, st);
             copyAsync(g.ckV + c * g.s.N, g.v, nb, st);
         }
-        runSubstep(g, g.x, g.v, false, st);
+        const cn_status r = step(g, own, st);
+        if (r != CN_OK) return r;
     }
     if (xOut) copyAsync(xOut, g.x, nb, st);
     if (vOut) copyAsync(vOut, g.v, nb, st);
@@ -573,14 +659,14 @@ template <class T> cn_status forward(Engine<T> &g, const T *compliance, const P4
 // derivative here: it only arises for tets whose four particles are all pinned (their records are
 // never applied) or whose denominator vanishes.
 template <class T> cn_status backward(Engine<T> &g, const P4<T> *gXOut, const P4<T> *gVOut, T *gCompliance,
-                                      P4<T> *gX0, P4<T> *gV0, cudaStream_t st)
+                                      P4<T> *gX0, P4<T> *gV0, cudaStream_t own, cudaStream_t st)
 {
     if (!g.forwardDone) return setError(CN_ERR_NOT_INITIALIZED, "cn_diff_backward: run cn_diff_forward first");
     const DScene<T> &s = g.s;
     const size_t nb = sizeof(P4<T>) * s.N;
     if (gXOut) copyAsync(g.gX, gXOut, nb, st); else cudaMemsetAsync(g.gX, 0, nb, st);
     if (gVOut) copyAsync(g.gV, gVOut, nb, st); else cudaMemsetAsync(g.gV, 0, nb, st);
-    if (s.T_) cudaMemsetAsync(gCompliance, 0, sizeof(T) * s.T_, st);
+    if (s.T_) cudaMemsetAsync(g.gCompliance, 0, sizeof(T) * s.T_, st);
     const uint32_t segments = (g.substeps + g.interval - 1) / g.interval;
     for (int seg = int(segments) - 1; seg >= 0; --seg) {
         const uint32_t first = uint32_t(seg) * g.interval;
@@ -593,38 +679,19 @@ template <class T> cn_status backward(Engine<T> &g, const P4<T> *gXOut, const P4
         for (uint32_t k = 0; k < count; ++k) {
             copyAsync(g.segX + size_t(k) * s.N, g.x, nb, st);
             copyAsync(g.segV + size_t(k) * s.N, g.v, nb, st);
-            if (k + 1 < count) runSubstep(g, g.x, g.v, false, st);
+            if (k + 1 < count) {
+                const cn_status r = step(g, own, st);
+                if (r != CN_OK) return r;
+            }
         }
         for (int k = int(count) - 1; k >= 0; --k) {
-            // this substep's iteration states
             copyAsync(g.x, g.segX + size_t(k) * s.N, nb, st);
             copyAsync(g.v, g.segV + size_t(k) * s.N, nb, st);
-            runSubstep(g, g.x, g.v, true, st);
-            // velocity update backwards: gA = adjoint entering the last iteration's output
-            k_dVelocityBack<T><<<gridOf(s.N), kDiffThreads, 0, st>>>(s, g.gX, g.gV, g.gA, g.dt);
-            if (s.E) cudaMemsetAsync(g.gLE, 0, sizeof(T) * s.E, st);
-            if (s.T_) cudaMemsetAsync(g.gLT, 0, sizeof(T) * s.T_, st);
-            for (int it = int(g.iterations) - 1; it >= 0; --it) {
-                if (s.T_) {
-                    k_dTetsBack<T><<<gridOf(s.T_), kDiffThreads, 0, st>>>(
-                        s, g.itX1 + size_t(it) * s.N, g.compliance, g.itLT + size_t(it) * s.T_, g.gA, g.gLT, g.recT,
-                        gCompliance, g.dt);
-                    k_dGather<T, 4><<<gridOf(s.N), kDiffThreads, 0, st>>>(s, g.gA, g.gB, s.tetRanges, s.tetInc,
-                                                                         g.recT);
-                    std::swap(g.gA, g.gB);
-                }
-                if (s.E) {
-                    k_dEdgesBack<T><<<gridOf(s.E), kDiffThreads, 0, st>>>(
-                        s, g.itX0 + size_t(it) * s.N, g.itLE + size_t(it) * s.E, g.gA, g.gLE, g.recE, g.dt);
-                    k_dGather<T, 2><<<gridOf(s.N), kDiffThreads, 0, st>>>(s, g.gA, g.gB, s.edgeRanges, s.edgeInc,
-                                                                         g.recE);
-                    std::swap(g.gA, g.gB);
-                }
-            }
-            // predict backwards: (gX, gV) of the substep start
-            k_dPredictBack<T><<<gridOf(s.N), kDiffThreads, 0, st>>>(s, g.gA, g.gV, g.gX, g.gV, g.dt);
+            const cn_status r = replay(g, g.adjointGraph, own, st, [](Engine<T> &e, cudaStream_t on) { runAdjoint(e, on); });
+            if (r != CN_OK) return r;
         }
     }
+    if (s.T_) cudaMemcpyAsync(gCompliance, g.gCompliance, sizeof(T) * s.T_, cudaMemcpyDefault, st);
     if (gX0) copyAsync(gX0, g.gX, nb, st);
     if (gV0) copyAsync(gV0, g.gV, nb, st);
     const cudaError_t e = cudaGetLastError();
@@ -678,8 +745,9 @@ template <class T> cn_status build(Engine<T> &g, const cn_world_soa &w, const cn
     uint32_t *den = g.template alloc<uint32_t>(E);
     uint4 *dtets = g.template alloc<uint4>(TT);
     T *dtrest = g.template alloc<T>(TT);
-    uint2 *eR = g.template alloc<uint2>(N), *eInc = g.template alloc<uint2>(eI.inc.size());
-    uint2 *tR = g.template alloc<uint2>(N), *tInc = g.template alloc<uint2>(tI.inc.size());
+    uint2 *eR = g.template alloc<uint2>(N), *tR = g.template alloc<uint2>(N);
+    uint32_t *eDst = g.template alloc<uint32_t>(eI.dst.size()), *tDst = g.template alloc<uint32_t>(tI.dst.size());
+    g.compliance = g.template alloc<T>(TT); g.gCompliance = g.template alloc<T>(TT);
     const size_t ck = g.substeps / g.interval + 1;
     g.x = g.template alloc<P4<T>>(N); g.v = g.template alloc<P4<T>>(N); g.xprev = g.template alloc<P4<T>>(N);
     g.lamE = g.template alloc<T>(E); g.lamT = g.template alloc<T>(TT);
@@ -696,9 +764,13 @@ template <class T> cn_status build(Engine<T> &g, const cn_world_soa &w, const cn
         if (!p) return setError(CN_ERR_OUT_OF_MEMORY, "cn_diff_set_scene: device allocation failed");
     upload(dw, wv); upload(ddamp, damp); upload(dpairs, pairs); upload(drest, rest); upload(decomp, ecomp);
     upload(den, en); upload(dtets, tets); upload(dtrest, trest);
-    upload(eR, eI.ranges); upload(eInc, eI.inc); upload(tR, tI.ranges); upload(tInc, tI.inc);
+    upload(eR, eI.ranges); upload(eDst, eI.dst); upload(tR, tI.ranges); upload(tDst, tI.dst);
+    // the first iteration starts from zero lambdas: the adjoint reads them in the first slots, which nothing writes
+    cudaMemset(g.itLE, 0, sizeof(T) * std::max<uint32_t>(E, 1u));
+    cudaMemset(g.itLT, 0, sizeof(T) * std::max<uint32_t>(TT, 1u));
     s.w = dw; s.damp = ddamp; s.edgePair = dpairs; s.edgeRest = drest; s.edgeCompliance = decomp; s.edgeEnabled = den;
-    s.tetIdx = dtets; s.tetRest = dtrest; s.edgeRanges = eR; s.edgeInc = eInc; s.tetRanges = tR; s.tetInc = tInc;
+    s.tetIdx = dtets; s.tetRest = dtrest; s.edgeRanges = eR; s.tetRanges = tR;
+    s.edgeDst = reinterpret_cast<const uint2 *>(eDst); s.tetDst = reinterpret_cast<const uint4 *>(tDst);
     const cudaError_t e = cudaDeviceSynchronize();
     if (e != cudaSuccess) return setError(CN_ERR_CUDA, std::string("cn_diff_set_scene: ") + cudaGetErrorString(e));
     return CN_OK;
@@ -796,10 +868,10 @@ CN_API cn_status cn_diff_forward(cn_diff *g, const void *tet_compliance, const v
     if (g->desc.precision == 8)
         return forward(g->f64, static_cast<const double *>(tet_compliance), static_cast<const P4<double> *>(x0),
                        static_cast<const P4<double> *>(v0), static_cast<P4<double> *>(x_out),
-                       static_cast<P4<double> *>(v_out), st);
+                       static_cast<P4<double> *>(v_out), g->ownStream, st);
     return forward(g->f32, static_cast<const float *>(tet_compliance), static_cast<const P4<float> *>(x0),
                    static_cast<const P4<float> *>(v0), static_cast<P4<float> *>(x_out), static_cast<P4<float> *>(v_out),
-                   st);
+                   g->ownStream, st);
 }
 
 CN_API cn_status cn_diff_backward(cn_diff *g, const void *grad_x_out, const void *grad_v_out, void *grad_tet_compliance,
@@ -812,10 +884,10 @@ CN_API cn_status cn_diff_backward(cn_diff *g, const void *grad_x_out, const void
     if (g->desc.precision == 8)
         return backward(g->f64, static_cast<const P4<double> *>(grad_x_out), static_cast<const P4<double> *>(grad_v_out),
                         static_cast<double *>(grad_tet_compliance), static_cast<P4<double> *>(grad_x0),
-                        static_cast<P4<double> *>(grad_v0), st);
+                        static_cast<P4<double> *>(grad_v0), g->ownStream, st);
     return backward(g->f32, static_cast<const P4<float> *>(grad_x_out), static_cast<const P4<float> *>(grad_v_out),
                     static_cast<float *>(grad_tet_compliance), static_cast<P4<float> *>(grad_x0),
-                    static_cast<P4<float> *>(grad_v0), st);
+                    static_cast<P4<float> *>(grad_v0), g->ownStream, st);
 }
 
 CN_API cn_status cn_diff_memory(cn_diff *g, uint64_t *bytes)
