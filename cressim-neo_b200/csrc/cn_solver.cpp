@@ -363,6 +363,7 @@ void layout(cn_solver *sv, cn::Arena &a, const cn_world_soa &w, const cn::Incide
         s.runComp = a.take<uint32_t>(N); s.runPos = a.take<uint32_t>(N);
         s.cvals = a.take<uint32_t>(N); s.cCell = a.take<int4>(N); s.cRun = a.take<uint32_t>(N);
         s.fluidMaxDelta = a.take<uint32_t>(64);
+        s.fluidIterations = sv->fluidIt;
         // Superset lists (k_fluidNeighborsDensity modes 1 and 2).  Without particle-particle
         // contacts fluid x is fixed over the iterations and the positions are double-buffered;
         // with them the gather records each iteration's largest move from the build positions P0.
@@ -370,7 +371,7 @@ void layout(cn_solver *sv, cn::Arena &a, const cn_world_soa &w, const cn::Incide
         s.sup = a.take<uint32_t>(size_t(N) * s.supCap);
         s.supCount = a.take<uint32_t>(N);
         if (!sv->fluidXMoves) s.Pb = a.take<float4>(N);
-        else s.P0 = a.take<float4>(N);
+        if (sv->fluidXMoves || sv->fluidIt > 1u + cn::fluidRebuildAhead(N)) s.P0 = a.take<float4>(N);
         s.maxNbr = sv->desc.max_fluid_neighborhood;
         s.nbr = a.take<uint32_t>(std::max<size_t>(size_t(N) * s.maxNbr, 1));
         s.nbrCount = a.take<uint32_t>(N);
