@@ -117,7 +117,7 @@ inline float fromBits(uint32_t u)
 constexpr uint64_t kBytesPerParticle = 3 * 16 + 6 * 4 + 16 + 2 * 8 + 2 * 4 + 8;
 constexpr uint64_t kBytesPerEdge = 16 + 4 + 2 * 16 + 2 * 4;
 constexpr uint64_t kBytesPerTet = 32 + 4 + 4 * 16 + 4 * 4;
-constexpr uint64_t kBytesPerBody = 18 * 16 + 8 + 8;
+constexpr uint64_t kBytesPerBody = 16 * 16 + 8 + 8;
 constexpr uint64_t kBytesPerCollider = 48 + 32 + 16 + 3 * 16 + 4 * 16 + 4 + 4;
 
 } // namespace
@@ -283,7 +283,6 @@ void layoutPool(cn_batch *b, cn::Arena &a)
     s.prevBodyPos = a.take<float4>(B); s.prevBodyRot = a.take<float4>(B);
     s.predBodyPos = a.take<float4>(B); s.predBodyRot = a.take<float4>(B);
     s.predBodyLin = a.take<float4>(B); s.predBodyAng = a.take<float4>(B);
-    s.prevBodyUnit = a.take<float4>(B); s.predBodyUnit = a.take<float4>(B);
     s.colAabbMin = a.take<float4>(C); s.colAabbMax = a.take<float4>(C);
     s.colFrame = a.take<float4>(size_t(C) * 4);
     s.colQueryOrder = a.take<uint32_t>(C);

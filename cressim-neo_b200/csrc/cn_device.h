@@ -222,7 +222,7 @@ struct Scene {
     const float4 *colMat = nullptr;
     float4 *prevBodyPos = nullptr, *prevBodyRot = nullptr;
     float4 *predBodyPos = nullptr, *predBodyRot = nullptr, *predBodyLin = nullptr, *predBodyAng = nullptr;
-    // without dynamic bodies: the predict's normalised orientations, for the contacts
+    // a single world without dynamic bodies: the predict's normalised orientations, for the contacts
     float4 *prevBodyUnit = nullptr, *predBodyUnit = nullptr;
     float4 *colAabbMin = nullptr, *colAabbMax = nullptr;
     // rigid-rigid contacts (scenes with dynamic bodies): LBVH over the query-order colliders, the

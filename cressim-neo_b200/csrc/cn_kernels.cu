@@ -142,7 +142,7 @@ __device__ __forceinline__ void rigidPredictBody(const Scene &s, float dt, float
         s.predBodyLin[b] = mk4(l, lin.w);
         s.predBodyAng[b] = ang;
     }
-    if (!s.hasDynamic) { // what the contacts normalise for every pair of every iteration
+    if (s.predBodyUnit) { // what the contacts normalise for every pair of every iteration
         s.prevBodyUnit[b] = qNormalize(q);
         s.predBodyUnit[b] = qNormalize(s.predBodyRot[b]);
     }
@@ -1809,7 +1809,8 @@ __device__ __forceinline__ void applyGatherAt(const Scene &s, const uint2 *range
 // order (the components are independent sums, so the bits are those of one thread's), sixteen records in
 // flight.  The range and the position are read ahead of the wait -- a gather follows its family's
 // solve, which moves no particle and has itself waited for the kernel that last did -- so the records
-// are the one round trip after it.
+// are the one round trip after it (with the solves' loads ahead of the wait: the 16^3 cube's frame of 200
+// iterations 2.50 -> 1.75 ms).
 constexpr uint32_t kGatherLanes = 4u;
 constexpr uint32_t kGatherAhead = 16u;
 struct GatherLane {
@@ -2515,7 +2516,7 @@ struct ContactRange {
 __device__ __forceinline__ ContactRange contactRange(const Scene &s, uint32_t i)
 {
     ContactRange r{s.candCount[i], s.candOffset[i], 0u, 0u, 0u};
-    if (r.count == 0u) return r;
+    if (r.count == 0u || i < s.nProxy) return r; // a proxy particle has no contacts of its own here
     r.body = s.rigidPairs[min(r.first, s.rigidPairCapacity - 1u)].y; // past a full buffer: not used
     if (r.body >= s.B) return r;
     const uint2 cr = s.bodyColRanges[r.body];
@@ -2602,7 +2603,7 @@ __device__ __forceinline__ RigidContact generateRigidContact(const Scene &s, uin
         }
     }
     if (bestPen > 0.0f) {
-        const float4 bq = s.hasDynamic ? qNormalize(rot) : s.predBodyUnit[b];
+        const float4 bq = s.predBodyUnit ? s.predBodyUnit[b] : qNormalize(rot);
         out.particle = i; out.body = b; out.collider = bestCol; out.active = 1u;
         out.normalPenetration = mk4(bestN, bestPen);
         out.rigidLocalPoint = mk4(qInvRotate(bq, bestW - bpos), 0.0f);
@@ -2628,8 +2629,8 @@ __device__ __forceinline__ ContactBody loadContactBody(const Scene &s, uint32_t 
     ContactBody o;
     o.prevPos = s.prevBodyPos[b];
     o.predPos = s.predBodyPos[b];
-    o.prevQ = s.hasDynamic ? s.prevBodyRot[b] : s.prevBodyUnit[b];
-    o.predQ = s.hasDynamic ? s.predBodyRot[b] : s.predBodyUnit[b];
+    o.prevQ = s.predBodyUnit ? s.prevBodyUnit[b] : s.prevBodyRot[b];
+    o.predQ = s.predBodyUnit ? s.predBodyUnit[b] : s.predBodyRot[b];
     o.type = s.bodyType[b];
     return o;
 }
@@ -2643,8 +2644,8 @@ __device__ __forceinline__ ContactCorrection solveRigidContact(const Scene &s, c
     const float iS = sp.w;
     const f3 prevS = pt.prev;
     const float4 prevB = body.prevPos, predB = body.predPos;
-    const float4 prevQ = s.hasDynamic ? qNormalize(body.prevQ) : body.prevQ;
-    const float4 predQ = s.hasDynamic ? qNormalize(body.predQ) : body.predQ;
+    const float4 prevQ = s.predBodyUnit ? body.prevQ : qNormalize(body.prevQ);
+    const float4 predQ = s.predBodyUnit ? body.predQ : qNormalize(body.predQ);
     const float iR = body.type == CN_BODY_DYNAMIC ? predB.w : 0.0f;
     if (iS <= kEps && iR <= kEps) return out;
     const float pen = mn(mx(c.normalPenetration.w - cfg.slop, 0.0f), cfg.softMaxCorrection);
@@ -2710,6 +2711,10 @@ __device__ __forceinline__ f3 rigidContactsSum(const Scene &s, const Config &cfg
         for (uint32_t k = 0; k < range.count; ++k) {
             const uint32_t pi = range.first + k;
             if (pi >= lim) break;
+            if (pt.proxy) { // nothing but its (inactive) records
+                if (store) s.rigidContacts[pi] = RigidContact{};
+                continue;
+            }
             uint2 pr = make_uint2(i, range.body); // pairs are emitted particle-major
             uint32_t colliders = range.colliders, collider0 = range.collider;
             if (k) {
@@ -3919,8 +3924,9 @@ __global__ void __launch_bounds__(kBatchFusedThreads, 2) k_batchFusedIterations(
 // Resident coloured iterations: one CTA runs every iteration of a substep of a coloured schedule with
 // the scene's positions (and colour Jacobi's sums) in shared memory, a block barrier per colour.  A
 // colour of a small scene has fewer constraints than the CTA has threads, so a launch per colour is all
-// latency; here the next colour's records load while the current one is solved.  Per constraint the
-// same device functions, colours in the same order.
+// latency; here its edges, tets and lambdas sit in shared memory, 16 bytes an edge and 20 a tet.  Per
+// constraint the same device functions, colours in the same order.  990 particles, 4 substeps x 10
+// iterations: 6.35 -> 1.79 ms a frame; a step is now the ~250 dependent instructions of a tet.
 // ------------------------------------------------------------------------------------------
 constexpr uint32_t kColourThreads = 512u;
 
@@ -4472,7 +4478,7 @@ namespace {
 // particles: issue 43 %, long scoreboard 7.4 per issue, DRAM 13-20 % of peak).  Against the four per-family
 // launches an iteration it saves the correction records' trips through L2 (128 B a tet, 64 B an edge,
 // scattered) and two launches: 100K particles 3.97 -> 2.29 ms a frame of 80 iterations, a cloth of 12.5K
-// 1.29 -> 0.82 ms, 216 particles on the ground 1.24 -> 0.6 ms.
+// 1.32 -> 0.75 ms, 216 particles in contact 1.24 -> 0.66 ms.
 constexpr int kTileThreads = 256;
 constexpr int kTileBlocks = 2;
 constexpr int kTileAhead = 3;      // entries per thread loaded before the predecessor is waited for

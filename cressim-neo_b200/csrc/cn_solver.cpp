@@ -258,7 +258,8 @@ void layout(cn_solver *sv, cn::Arena &a, const cn_world_soa &w, const cn::Incide
     s.prevBodyPos = a.take<float4>(B); s.prevBodyRot = a.take<float4>(B);
     s.predBodyPos = a.take<float4>(B); s.predBodyRot = a.take<float4>(B);
     s.predBodyLin = a.take<float4>(B); s.predBodyAng = a.take<float4>(B);
-    s.prevBodyUnit = a.take<float4>(B); s.predBodyUnit = a.take<float4>(B);
+    s.prevBodyUnit = sv->hasDynamic ? nullptr : a.take<float4>(B);
+    s.predBodyUnit = sv->hasDynamic ? nullptr : a.take<float4>(B);
     s.colAabbMin = a.take<float4>(C); s.colAabbMax = a.take<float4>(C);
     s.nProxy = sv->nProxy;
     s.proxyLocal = a.take<float4>(sv->nProxy);
@@ -910,7 +911,11 @@ static void buildSolverTiles(cn_solver *sv, const cn_world_soa &w, const cn::Inc
     sv->tileContacts = contacts;
     const uint32_t target = cn::tileTarget(N);
     if (!target) return;
-    sv->tileBuild = cn::buildTiles(in, target, cn::kTileSmemCap);
+    try {
+        sv->tileBuild = cn::buildTiles(in, target, cn::kTileSmemCap);
+    } catch (const std::exception &) { // no memory for the lists: the per-family kernels run
+        sv->tileBuild = cn::TileBuild{};
+    }
     if (sv->tileBuild.ok && !cn::tileKernelsFit(cn::kTileSmemCap)) sv->tileBuild = cn::TileBuild{};
 }
 
