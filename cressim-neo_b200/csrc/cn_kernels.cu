@@ -1175,7 +1175,10 @@ __global__ void __launch_bounds__(kFluidThreads, (kExtras ? 4 : 5) * (256 / kFlu
     if (Dk) reinterpret_cast<float *>(Dk + slot)[3] = C;
 }
 
-// What a particle brings to its pair terms of the position delta.
+// The pair term, the boundary part and the apply of the position delta as functions, for k_fluidDeltaWide.
+// k_fluidDeltaApplyClamp below holds the same expressions in its body: through these its register allocation
+// comes out 1 % slower at 1M particles.
+// What a particle brings to its pair terms.
 struct FluidSelf {
     f3 sp, sdl, sn;
     float sC, h, kW, invH, cohesion, c1, c2, visc, st, cfl, dt;
@@ -1335,7 +1338,18 @@ __global__ void __launch_bounds__(kFluidThreads, (kExtras ? 4 : 5) * (256 / kFlu
     f3 packed{0.f, 0.f, 0.f};
     float weight = 0.0f;
     if (__float_as_uint(self.w) & kFluidBit) {
-        const FluidSelf me = fluidSelf<kExtras>(s, fm, self, sdl, s.Cs[slot], myMat, dt);
+        const f3 sp = xyz(self);
+        const float4 snc = s.Cs[slot];
+        const float sC = snc.w;
+        const float h = mx(fm.smoothing_radius, 1.0e-4f);
+        const float kW = spikyK(h);
+        const float invH = 1.0f / h;
+        const float cohesion = kExtras ? dt * mx(fm.cohesion, 0.0f) : 0.0f;
+        const float visc = dt * mx(fm.viscosity, 0.0f);
+        const float st = kExtras ? mx(fm.surface_tension, 0.0f) : 0.0f;
+        const float cfl = mx(fm.cfl_radius, 0.0f);
+        const bool needRel = visc > kEps || cfl > kEps;
+        const f3 sn = st > kEps ? xyz(snc) : f3{0.f, 0.f, 0.f};
         f3 dp{0.f, 0.f, 0.f};
         const uint32_t cnt = s.nbrCount[slot];
         // 32-bit list offsets (N x max neighbours < 2^32 is checked at sync)
@@ -1353,6 +1367,7 @@ __global__ void __launch_bounds__(kFluidThreads, (kExtras ? 4 : 5) * (256 / kFlu
         for (uint32_t k = 0; k < cnt; ++k) {
             const uint32_t c = cN;
             const float4 np = npN;
+            const float ncw = dN.w;
             const float4 nd4 = dN;
             if (k + 1 < cnt) {
                 cN = cNN;
@@ -1360,14 +1375,86 @@ __global__ void __launch_bounds__(kFluidThreads, (kExtras ? 4 : 5) * (256 / kFlu
                 npN = ld4(&s.P[cN]);
                 dN = ld4(&Dcur[cN]);
             }
-            f3 pd;
-            if (!fluidPair<kExtras>(s, me, iter, np, nd4, c, pd)) continue;
+            const uint32_t tag = __float_as_uint(np.w);
+            if ((tag & kFluidBit) == 0u) continue;
+            const f3 delta = sp - xyz(np);
+            const float dist = length(delta);
+            if (dist >= h || dist <= kEps) continue;
+            const f3 nij = delta * (1.0f / dist);
+            // spikyDW / spikyW of physics_fluid_common.hlsli:17-41 sharing 1 - dist / h
+            const float om = 1.0f - dist * invH;
+            const float dw = -2.0f * kW * om * invH;
+            f3 pd = -0.5f * (sC + ncw) * dw * nij;
+            if (infoMaterial(tag) == myMat) {
+                if (kExtras && cohesion > kEps)
+                    pd -= nij * (cohesion * cohesionW(dist, h, invH, fm.cohesion1, fm.cohesion2));
+                if (needRel) {
+                    const f3 nd = iter > 0 ? xyz(nd4) : f3{0.f, 0.f, 0.f};
+                    const f3 rel = sdl - nd;
+                    if (visc > kEps) {
+                        const float vs = 1.0f - (1.0f / (1.0f + visc * (kW * om * om)));
+                        pd -= vs * rel;
+                    }
+                    if (cfl > kEps) {
+                        const float proj = dot(rel, nij);
+                        if (proj < -cfl) pd -= nij * (proj + cfl) * 0.5f;
+                    }
+                }
+                if (kExtras && st > kEps) pd -= dt * (sn - xyz(ld4(&s.Cs[c])));
+            }
             dp += pd;
             weight += 1.0f;
         }
-        packed = dp * cfg.fluidSolveCoefficient + fluidBoundaryDelta(s, cfg, slot, me);
+        f3 bd{0.f, 0.f, 0.f};
+        forEachBoundary(s, slot, [&](uint32_t k) {
+            f3 ghost;
+            if (!fluidGhostDelta(s, s.colQueryOrder[k], sp, h, ghost)) return;
+            const float dist = length(ghost);
+            if (dist <= kEps || dist >= h) return;
+            const f3 nij = ghost * (1.0f / dist);
+            const float dw = spikyDWk(dist, h, invH, kW);
+            bd += -mx(sC, 0.0f) * dw * nij;
+        });
+        bd = bd * cfg.fluidBoundaryDeltaScale;
+        packed = dp * cfg.fluidSolveCoefficient + bd;
     }
-    fluidApplyClamp(s, cfg, slot, self, sdl, packed, weight, Xs, Dnext, Pnext, iter, writeDx);
+    if (writeDx) s.Dx[slot] = mk4(packed, weight);
+    // apply (physics_fluid_apply_delta_positions.cs.hlsl:21-30)
+    const float w = mx(weight * cfg.fluidRelaxation, 1.0f);
+    const f3 d = packed / w;
+    const f3 acc = sdl + d;
+    // clamp (physics_fluid_clamp_boundary.cs.hlsl:36-79)
+    const f3 base = xyz(Xs[slot]);
+    f3 cur = base + acc;
+    if (hasBoundary(s, slot)) {
+        const uint32_t p = s.cvals[slot];
+        const float pr = mx(s.radii[p], 0.0f);
+        for (uint32_t sweep = 0; sweep < 2u; ++sweep) {
+            bool changed = false;
+            forEachBoundary(s, slot, [&](uint32_t k) {
+                float sd = 0.0f;
+                f3 n{0.f, 1.f, 0.f};
+                if (!fluidBoundaryContactInfo(s, s.colQueryOrder[k], cur, sd, n)) return;
+                if (sd >= pr) return;
+                cur += n * (pr - sd);
+                changed = true;
+            });
+            if (!changed) break;
+        }
+    }
+    const f3 dn = cur - base;
+    Dnext[slot] = mk4(dn, 0.0f);
+    if (Pnext) {
+        Pnext[slot] = mk4(base + dn, self.w);
+        const uint32_t next = iter + 1u;
+        if (next < kMaxTrackedIterations) {
+            // lanes that returned early are not in the mask; diverged groups reduce separately
+            const f3 moved = s.P0 ? (base + dn) - xyz(s.P0[slot]) : dn;
+            const unsigned mask = __activemask();
+            const uint32_t big = __reduce_max_sync(mask, __float_as_uint(sqrtf(dot(moved, moved))));
+            if (int(threadIdx.x & 31u) == __ffs(mask) - 1 && big > 0u) atomicMax(&s.fluidMaxDelta[next], big);
+        }
+    }
 }
 
 // The two fluid kernels for scenes that leave most of the chip idle with a thread per particle: kLanes
