@@ -114,3 +114,12 @@ def test_restitution_after_the_iterations():
     w.velocities()[:, 1] = np.float32(-3.0)
     desc = solver_desc(substeps=2, default_iterations=6, enable_blocking_readback=0)
     _equal(*_states(w, desc, 4))
+
+
+@pytest.mark.parametrize("schedule", [1, 2])
+def test_resident_colours_with_a_particle_named_twice(schedule):
+    w = _block((4, 4, 4), pinned=False)
+    w.array("tets")[::5, 3] = w.array("tets")[::5, 1]
+    desc = solver_desc(substeps=2, default_iterations=3, enable_blocking_readback=0)
+    desc.soft.xpbd_schedule = schedule
+    _equal(*_states(w, desc))
