@@ -721,11 +721,12 @@ def run_diff(stream, cpu_sample: bool = True) -> dict:
     g = torch.zeros_like(x0)
     g[surf, :3] = 1e-3
     gc, gv = torch.zeros_like(comp), torch.zeros_like(v0)
-    ev[0].record(stream)
-    r.forward(comp, x0, v0, out)
-    ev[1].record(stream)
-    r.backward(g, None, gc, None, gv)
-    ev[2].record(stream)
+    with torch.cuda.stream(stream):  # the rollout runs on torch's current stream: the events belong on the same one
+        ev[0].record(stream)
+        r.forward(comp, x0, v0, out)
+        ev[1].record(stream)
+        r.backward(g, None, gc, None, gv)
+        ev[2].record(stream)
     torch.cuda.synchronize()
     fwd_ms, bwd_ms = ev[0].elapsed_time(ev[1]), ev[1].elapsed_time(ev[2])
     kept = r.memory_bytes()
