@@ -329,6 +329,7 @@ struct Scene {
     uint32_t *supCount = nullptr;     // per sorted slot (> supCap: overflowed)
     uint32_t *fluidMaxDelta = nullptr; // [64] float bits of max |accumulated delta| per iteration
     uint32_t fluidIterations = 0;     // of a substep
+    const float *fluidMinRadius = nullptr; // least smoothing radius of the fluid materials
     float4 *fluidVort = nullptr;      // curl xyz + magnitude per sorted slot (vorticity confinement)
 
     // ---- contact candidates ----

@@ -984,6 +984,14 @@ __device__ __forceinline__ bool neighborAllowed(const Scene &s, uint32_t tag, ui
     return om.x == m.x && (m.w & om.z) != 0u && (om.w & m.z) != 0u;
 }
 
+// Whether an iteration builds the superset lists anew: all of the scene's or none (fluids of several
+// smoothing radii have several bounds).  A list holds while its particle's candidates have moved less than
+// the margin since it was recorded, and their moves are measured from the positions of their own build.
+__device__ __forceinline__ bool supersetsAnew(const Scene &s, float maxDelta)
+{
+    return !(2.0f * maxDelta < 0.99f * s.supMargin * __ldg(s.fluidMinRadius));
+}
+
 // Neighbour list + density constraint.
 // physics_fluid_build_neighbors.cs.hlsl:21-147 fused with
 // physics_fluid_compute_density_lambda.cs.hlsl:26-115.  The density sum runs over the list in
@@ -1001,9 +1009,10 @@ __device__ __forceinline__ bool neighborAllowed(const Scene &s, uint32_t tag, ui
 //         margin * h every neighbour of this iteration is in the superset, and filtering it in order
 //         yields exactly the list the cell walk would build.  Otherwise (or if this particle's
 //         superset overflowed) the particle walks the cells.
-// mode 4: as mode 2, but where the moves are over the bound the walk records the superset anew, with the
-//         positions the moves are measured from (P0), as mode 1 does: a fluid that moves far early in
-//         a substep -- a compressed block, a splash -- filters again in the iterations that follow.
+// mode 4: as mode 2, but where the moves are over the bound of the least smoothing radius every particle
+//         walks and records the superset anew, with the positions the moves are measured from (P0), as
+//         mode 1 does: a fluid that moves far early in a substep -- a compressed block, a splash --
+//         filters again in the iterations that follow.
 // One instantiation per mode, so the cell walk's register needs do not set the filter's occupancy;
 // the filter is held to 64 registers (4 blocks of 256 per SM: 14 % faster than 65 registers and
 // 3 blocks, measured; 48 registers and 5 blocks spill).
@@ -1051,8 +1060,8 @@ __global__ void __launch_bounds__(kFluidThreads, (kExtras ? 4 : 5) * (256 / kFlu
     if (mode == 2u || mode == 4u) {
         const float maxDelta = __uint_as_float(s.fluidMaxDelta[iter < kMaxTrackedIterations ? iter : 0u]);
         const bool holds = iter < kMaxTrackedIterations && 2.0f * maxDelta < 0.99f * s.supMargin * h;
-        useSuperset = holds && s.supCount[slot] <= s.supCap;
-        rebuild = mode == 4u && !holds && iter + 1u < kMaxTrackedIterations;
+        rebuild = mode == 4u && iter + 1u < kMaxTrackedIterations && supersetsAnew(s, maxDelta);
+        useSuperset = holds && !rebuild && s.supCount[slot] <= s.supCap;
     }
     if (useSuperset) {
         const uint32_t n = s.supCount[slot];
@@ -1554,8 +1563,8 @@ __global__ void __launch_bounds__(kFluidThreads) k_fluidNeighborsWide(Scene s, C
     if (mode != 3u) {
         const float maxDelta = __uint_as_float(s.fluidMaxDelta[iter < kMaxTrackedIterations ? iter : 0u]);
         const bool holds = iter < kMaxTrackedIterations && 2.0f * maxDelta < 0.99f * s.supMargin * h;
-        useSuperset = holds && s.supCount[slot] <= s.supCap;
-        rebuild = mode == 4u && !holds && iter + 1u < kMaxTrackedIterations;
+        rebuild = mode == 4u && iter + 1u < kMaxTrackedIterations && supersetsAnew(s, maxDelta);
+        useSuperset = holds && !rebuild && s.supCount[slot] <= s.supCap;
     }
     if (useSuperset) {
         const uint32_t n = s.supCount[slot];

@@ -95,6 +95,7 @@ struct cn_solver {
     cn::TileBuild tileBuild;
     cn::TileSet tiles{};
     bool tileContacts = false;
+    float fluidMinRadius = 0.0f; // of Scene::fluidMinRadius, kept while its upload runs
     bool residentColour = false; // a coloured schedule's iterations in one CTA
 };
 
@@ -365,6 +366,7 @@ void layout(cn_solver *sv, cn::Arena &a, const cn_world_soa &w, const cn::Incide
         s.cvals = a.take<uint32_t>(N); s.cCell = a.take<int4>(N); s.cRun = a.take<uint32_t>(N);
         s.fluidMaxDelta = a.take<uint32_t>(64);
         s.fluidIterations = sv->fluidIt;
+        s.fluidMinRadius = a.take<float>(1);
         // Superset lists (k_fluidNeighborsDensity modes 1 and 2).  Without particle-particle
         // contacts fluid x is fixed over the iterations and the positions are double-buffered;
         // with them the gather records each iteration's largest move from the build positions P0.
@@ -461,6 +463,17 @@ cn_status uploadSurfaceRender(cn_solver *sv, const cn_world_soa &w, cudaStream_t
     CN_CUDA(up(s.surfChunkRange, ranges.data(), ranges.size(), st));
     CN_CUDA(cudaStreamSynchronize(st)); // the host tables above go out of scope
     return CN_OK;
+}
+
+// The fluid materials and the least of their smoothing radii, as the kernels read a radius.
+cudaError_t uploadFluidMaterials(cn_solver *sv, const cn_world_soa &w, cudaStream_t st)
+{
+    const cudaError_t e = up(sv->s.fluidMaterials, w.fluid_materials, w.fluid_material_count, st);
+    if (e != cudaSuccess || !sv->s.fluidMinRadius || !w.fluid_material_count) return e;
+    float least = w.fluid_materials[0].smoothing_radius;
+    for (uint32_t m = 1; m < w.fluid_material_count; ++m) least = std::min(least, w.fluid_materials[m].smoothing_radius);
+    sv->fluidMinRadius = std::max(least, 1.0e-4f);
+    return up(sv->s.fluidMinRadius, &sv->fluidMinRadius, 1, st);
 }
 
 constexpr uint32_t kTileFams = (1u << cn::kFamEdges) | (1u << cn::kFamBends) | (1u << cn::kFamTets);
@@ -1172,7 +1185,7 @@ CN_API cn_status cn_solver_sync_world(cn_solver *sv, const cn_world_soa *w)
     CN_CUDA(up(s.adjCnt, w->adjacency_counts, N, st));
     CN_CUDA(up(s.adjIdx, w->adjacency_indices, w->adjacency_index_count, st));
     CN_CUDA(up(s.contactMaterials, w->contact_materials, w->contact_material_count, st));
-    CN_CUDA(up(s.fluidMaterials, w->fluid_materials, w->fluid_material_count, st));
+    CN_CUDA(uploadFluidMaterials(sv, *w, st));
     CN_CUDA(up(s.edges, w->edges, s.E, st));
     CN_CUDA(up(s.bends, w->bends, s.Bn, st));
     CN_CUDA(up(s.dihedrals, w->dihedrals, s.D, st));
@@ -1553,7 +1566,7 @@ CN_API cn_status cn_solver_update_world(cn_solver *sv, const cn_world_soa *w, ui
         CN_CUDA(up(s.matIdx, w->material_indices, N, st));
         CN_CUDA(up(s.fluidMatIdx, w->fluid_material_indices, N, st));
         CN_CUDA(up(s.contactMaterials, w->contact_materials, w->contact_material_count, st));
-        CN_CUDA(up(s.fluidMaterials, w->fluid_materials, w->fluid_material_count, st));
+        CN_CUDA(uploadFluidMaterials(sv, *w, st));
         if (s.nProxy) CN_CUDA(up(s.proxyLocal, w->rigid_proxy_local_positions, s.nProxy, st));
     }
     if (flags & CN_SYNC_CONSTRAINTS) {
