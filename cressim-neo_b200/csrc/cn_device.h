@@ -328,6 +328,9 @@ struct Scene {
     uint32_t *sup = nullptr;          // [N][supCap] candidates within the superset radius, traversal order
     uint32_t *supCount = nullptr;     // per sorted slot (> supCap: overflowed)
     uint32_t *fluidMaxDelta = nullptr; // [64] float bits of max |accumulated delta| per iteration
+    // [64] each: whether an iteration of this substep built the superset anew ([0]: any did); whether the
+    // lists it built last did not last (kept over the substeps: it decides what is tried, not what results)
+    uint32_t *fluidBuilt = nullptr, *fluidOvertaken = nullptr;
     uint32_t fluidIterations = 0;     // of a substep
     const float *fluidMinRadius = nullptr; // least smoothing radius of the fluid materials
     float4 *fluidVort = nullptr;      // curl xyz + magnitude per sorted slot (vorticity confinement)
@@ -456,9 +459,10 @@ void launchFluidIteration(const Scene &s, uint32_t iter, float dt, const Config 
                           cudaStream_t st);
 void launchFluidGather(const Scene &s, uint32_t iter, cudaStream_t st);
 // Iterations that have to follow for the superset lists to be built anew where the moves are over their bound:
-// the walk that records them costs about one and a half times the walk that does not (4 iterations: a
-// 120K-particle block 1.39 -> 1.36 ms a frame with two, 1M particles 5.58 -> 5.77).
-inline uint32_t fluidRebuildAhead(uint32_t n) { return n < 262144u ? 2u : 4u; }
+// recording them costs about half a walk of the cells, which two filters in place of walks repay (4
+// iterations: a 480K-particle splash 3,490 -> 3,220 us a frame, 1M particles 6,940 -> 6,610; a fluid at rest
+// the same).
+constexpr uint32_t kFluidRebuildAhead = 2u;
 // False when the positions are double-buffered: the gather then runs at the first iteration only.
 bool fluidGatherEachIteration(const Scene &s);
 // walkCells: every iteration walks the 27 cells (no superset lists).

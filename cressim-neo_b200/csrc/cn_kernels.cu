@@ -987,9 +987,31 @@ __device__ __forceinline__ bool neighborAllowed(const Scene &s, uint32_t tag, ui
 // Whether an iteration builds the superset lists anew: all of the scene's or none (fluids of several
 // smoothing radii have several bounds).  A list holds while its particle's candidates have moved less than
 // the margin since it was recorded, and their moves are measured from the positions of their own build.
-__device__ __forceinline__ bool supersetsAnew(const Scene &s, float maxDelta)
+// Built anew where the moves are over the bound.  An iteration whose lists did not last through the next two
+// (noteSuperset) leaves it, in the substeps that follow, until the move since the last iteration is below
+// the bound for two: a fluid that outruns its lists every time only pays for recording them (4 iterations,
+// late frames of a 262K-particle gas 2,400 us a frame without, 2,530 with, a pressed block of 110K 5,050 and 5,560).
+__device__ __forceinline__ bool supersetsAnew(const Scene &s, uint32_t iter)
 {
-    return !(2.0f * maxDelta < 0.99f * s.supMargin * __ldg(s.fluidMinRadius));
+    const float moved = __uint_as_float(s.fluidMaxDelta[iter]), bound = 0.99f * s.supMargin * __ldg(s.fluidMinRadius);
+    if (2.0f * moved < bound) return false;
+    if (s.fluidOvertaken[iter] == 0u) return true;
+    const bool fresh = iter == 1u || s.fluidBuilt[iter - 1u] != 0u;
+    return (fresh ? moved : moved - __uint_as_float(s.fluidMaxDelta[iter - 1u])) < bound;
+}
+__device__ __forceinline__ void supersetBuilt(const Scene &s, uint32_t iter)
+{
+    s.fluidBuilt[iter] = 1u;
+    s.fluidBuilt[0] = 1u;
+}
+
+// After a substep's iterations: whether the lists that iteration k built lasted through the next two.
+__device__ __forceinline__ void noteSuperset(const Scene &s, uint32_t k)
+{
+    if (k == 0u || k + kFluidRebuildAhead >= s.fluidIterations || k + kFluidRebuildAhead >= kMaxTrackedIterations || s.fluidBuilt[k] == 0u) return;
+    const float bound = 0.99f * s.supMargin * __ldg(s.fluidMinRadius);
+    const float moved = fmaxf(__uint_as_float(s.fluidMaxDelta[k + 1u]), __uint_as_float(s.fluidMaxDelta[k + kFluidRebuildAhead]));
+    s.fluidOvertaken[k] = s.fluidBuilt[k + 1u] == 0u && 2.0f * moved < bound ? 0u : 1u;
 }
 
 // Neighbour list + density constraint.
@@ -1009,10 +1031,10 @@ __device__ __forceinline__ bool supersetsAnew(const Scene &s, float maxDelta)
 //         margin * h every neighbour of this iteration is in the superset, and filtering it in order
 //         yields exactly the list the cell walk would build.  Otherwise (or if this particle's
 //         superset overflowed) the particle walks the cells.
-// mode 4: as mode 2, but where the moves are over the bound of the least smoothing radius every particle
-//         walks and records the superset anew, with the positions the moves are measured from (P0), as
-//         mode 1 does: a fluid that moves far early in a substep -- a compressed block, a splash --
-//         filters again in the iterations that follow.
+// k_fluidFilterAnew is mode 2 for scenes of more iterations: where the moves are over the bound of the least
+//         smoothing radius every particle first records its superset anew, with the position its moves
+//         are then measured from (P0), as mode 3 does: a fluid that moves far early in a substep -- a
+//         compressed block, a splash -- filters again in the iterations that follow.
 // One instantiation per mode, so the cell walk's register needs do not set the filter's occupancy;
 // the filter is held to 64 registers (4 blocks of 256 per SM: 14 % faster than 65 registers and
 // 3 blocks, measured; 48 registers and 5 blocks spill).
@@ -1022,12 +1044,9 @@ __device__ __forceinline__ bool supersetsAnew(const Scene &s, float maxDelta)
 // (fewer live registers: the kernels then run at 5 blocks of 256 per SM without spills -- the
 // filter 10 %, the superset build 5 % faster than the full build, measured).
 template <uint32_t mode, bool kExtras>
-__global__ void __launch_bounds__(kFluidThreads, (kExtras ? 4 : 5) * (256 / kFluidThreads)) k_fluidNeighborsDensity(Scene s, Config cfg, bool density,
-                                                                                    uint32_t iter, float4 *Dk)
+__device__ __forceinline__ void fluidNeighborsAt(const Scene &s, const Config &cfg, bool density, uint32_t iter, float4 *Dk,
+                                                 uint32_t slot, bool anew)
 {
-    pdlEnter();
-    const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
-    if (slot >= s.N) return;
     const uint32_t info = s.sInfo[slot];
     if ((info & kFluidBit) == 0u) {
         if (density && mode != 3u) s.Cs[slot] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1056,12 +1075,11 @@ __global__ void __launch_bounds__(kFluidThreads, (kExtras ? 4 : 5) * (256 / kFlu
     float rho = 0.0f;
     f3 normal{0.f, 0.f, 0.f};
 
-    bool useSuperset = false, rebuild = false;
-    if (mode == 2u || mode == 4u) {
+    bool useSuperset = false;
+    if (mode == 2u) {
         const float maxDelta = __uint_as_float(s.fluidMaxDelta[iter < kMaxTrackedIterations ? iter : 0u]);
-        const bool holds = iter < kMaxTrackedIterations && 2.0f * maxDelta < 0.99f * s.supMargin * h;
-        rebuild = mode == 4u && iter + 1u < kMaxTrackedIterations && supersetsAnew(s, maxDelta);
-        useSuperset = holds && !rebuild && s.supCount[slot] <= s.supCap;
+        const bool holds = anew || (iter < kMaxTrackedIterations && 2.0f * maxDelta < 0.99f * s.supMargin * h);
+        useSuperset = holds && s.supCount[slot] <= s.supCap;
     }
     if (useSuperset) {
         const uint32_t n = s.supCount[slot];
@@ -1095,7 +1113,7 @@ __global__ void __launch_bounds__(kFluidThreads, (kExtras ? 4 : 5) * (256 / kFlu
         const uint32_t myGroup = infoGroup(info);
         const bool selfCompat = (m.w & m.z) != 0u;
         const int4 e = s.cCell[slot];
-        const bool buildSup = mode == 1u || mode == 3u || rebuild;
+        const bool buildSup = mode == 1u || mode == 3u;
         const float supR = h * (1.0f + s.supMargin);
         const float sup2 = supR * supR;
         const float rec2 = buildSup ? (sup2 > h2 ? sup2 : h2) : h2;
@@ -1160,7 +1178,6 @@ __global__ void __launch_bounds__(kFluidThreads, (kExtras ? 4 : 5) * (256 / kFlu
                     }
                 }
         if (buildSup) s.supCount[slot] = supN; // > supCap marks an overflowed superset
-        if (rebuild) s.P0[slot] = self;
         if (mode == 3u) return;
     }
     s.nbrCount[slot] = count;
@@ -1182,6 +1199,45 @@ __global__ void __launch_bounds__(kFluidThreads, (kExtras ? 4 : 5) * (256 / kFlu
         s.Cs[slot] = make_float4(0.f, 0.f, 0.f, C);
     }
     if (Dk) reinterpret_cast<float *>(Dk + slot)[3] = C;
+}
+
+template <uint32_t mode, bool kExtras>
+__global__ void __launch_bounds__(kFluidThreads, (kExtras ? 4 : 5) * (256 / kFluidThreads)) k_fluidNeighborsDensity(Scene s, Config cfg, bool density,
+                                                                                    uint32_t iter, float4 *Dk)
+{
+    pdlEnter();
+    const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
+    if (slot >= s.N) return;
+    fluidNeighborsAt<mode, kExtras>(s, cfg, density, iter, Dk, slot, false);
+}
+
+// Records a particle's superset anew.  Not inlined: with the walk in its body the filter spills at 48
+// registers, or loses its loads in flight, and scenes that never build anew pay for it (20 iterations,
+// 512K particles at rest: 8,530 us a frame so, 8,940 with one walk for both lists, 9,000 inlined).
+template <bool kExtras> __device__ __noinline__ void recordSuperset(const Scene &s, const Config &cfg, uint32_t slot)
+{
+    // a warp with an overflowed list among its own would filter and walk: it walks until the next substep
+    if (__any_sync(__activemask(), s.supCount[slot] > s.supCap)) {
+        s.supCount[slot] = s.supCap + 1u;
+        return;
+    }
+    fluidNeighborsAt<3u, kExtras>(s, cfg, false, 0u, nullptr, slot, false);
+}
+
+template <bool kExtras>
+__global__ void __launch_bounds__(kFluidThreads, (kExtras ? 4 : 5) * (256 / kFluidThreads))
+    k_fluidFilterAnew(const __grid_constant__ Scene s, const __grid_constant__ Config cfg, uint32_t iter, float4 *Dk)
+{
+    pdlEnter();
+    const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
+    if (slot >= s.N) return;
+    const bool anew = iter + 1u < kMaxTrackedIterations && supersetsAnew(s, iter);
+    if (anew) {
+        supersetBuilt(s, iter);
+        s.P0[slot] = s.P[slot];
+        recordSuperset<kExtras>(s, cfg, slot);
+    }
+    fluidNeighborsAt<2u, kExtras>(s, cfg, true, iter, Dk, slot, anew);
 }
 
 // The pair term, the boundary part and the apply of the position delta as functions, for k_fluidDeltaWide.
@@ -1305,7 +1361,7 @@ __device__ __forceinline__ void fluidApplyClamp(const Scene &s, const Config &cf
         const uint32_t next = iter + 1u;
         if (next < kMaxTrackedIterations) {
             // lanes that returned early are not in the mask; diverged groups reduce separately
-            const f3 moved = s.P0 ? (base + dn) - xyz(s.P0[slot]) : dn;
+            const f3 moved = s.P0 && s.fluidBuilt[0] != 0u ? (base + dn) - xyz(s.P0[slot]) : dn;
             const unsigned mask = __activemask();
             const uint32_t big = __reduce_max_sync(mask, __float_as_uint(sqrtf(dot(moved, moved))));
             if (int(threadIdx.x & 31u) == __ffs(mask) - 1 && big > 0u) atomicMax(&s.fluidMaxDelta[next], big);
@@ -1458,7 +1514,7 @@ __global__ void __launch_bounds__(kFluidThreads, (kExtras ? 4 : 5) * (256 / kFlu
         const uint32_t next = iter + 1u;
         if (next < kMaxTrackedIterations) {
             // lanes that returned early are not in the mask; diverged groups reduce separately
-            const f3 moved = s.P0 ? (base + dn) - xyz(s.P0[slot]) : dn;
+            const f3 moved = s.P0 && s.fluidBuilt[0] != 0u ? (base + dn) - xyz(s.P0[slot]) : dn;
             const unsigned mask = __activemask();
             const uint32_t big = __reduce_max_sync(mask, __float_as_uint(sqrtf(dot(moved, moved))));
             if (int(threadIdx.x & 31u) == __ffs(mask) - 1 && big > 0u) atomicMax(&s.fluidMaxDelta[next], big);
@@ -1471,7 +1527,7 @@ __global__ void __launch_bounds__(kFluidThreads, (kExtras ? 4 : 5) * (256 / kFlu
 // evaluated side by side; the sums and the list positions then run over the lanes in list order, so
 // lists and sums are the ones of the kernels above.  A thread's serial chain (a gather, a square root and
 // two divisions per neighbour, some thousand cycles) is what bounds a small scene.
-// mode 2, 3, 4: as k_fluidNeighborsDensity.
+// mode 2, 3: as k_fluidNeighborsDensity; mode 4: as k_fluidFilterAnew, in one walk for both lists.
 template <uint32_t kLanes> struct LaneGroup {
     uint32_t lane, mask, shift;
     __device__ __forceinline__ LaneGroup()
@@ -1563,7 +1619,7 @@ __global__ void __launch_bounds__(kFluidThreads) k_fluidNeighborsWide(Scene s, C
     if (mode != 3u) {
         const float maxDelta = __uint_as_float(s.fluidMaxDelta[iter < kMaxTrackedIterations ? iter : 0u]);
         const bool holds = iter < kMaxTrackedIterations && 2.0f * maxDelta < 0.99f * s.supMargin * h;
-        rebuild = mode == 4u && iter + 1u < kMaxTrackedIterations && supersetsAnew(s, maxDelta);
+        rebuild = mode == 4u && iter + 1u < kMaxTrackedIterations && supersetsAnew(s, iter);
         useSuperset = holds && !rebuild && s.supCount[slot] <= s.supCap;
     }
     if (useSuperset) {
@@ -1636,7 +1692,10 @@ __global__ void __launch_bounds__(kFluidThreads) k_fluidNeighborsWide(Scene s, C
                 }
             }
         if (buildSup && writer) s.supCount[slot] = supN; // > supCap marks an overflowed superset
-        if (rebuild && writer) s.P0[slot] = self;
+        if (rebuild && writer) {
+            s.P0[slot] = self;
+            supersetBuilt(s, iter);
+        }
         if (mode == 3u) return;
     }
     truncated = group.ballot(truncated != 0u);
@@ -2956,6 +3015,7 @@ __device__ __forceinline__ void updateVelocityAt(const Scene &s, float dt, const
 __global__ void __launch_bounds__(kThreads) k_updateVelocities(Scene s, float dt, const float4 *Dfinal)
 {
     pdlEnter();
+    if (s.P0 && blockIdx.x == 0u && threadIdx.x < kMaxTrackedIterations) noteSuperset(s, threadIdx.x);
     forEachElem(s.wP, s.N, [&](uint32_t i) { updateVelocityAt(s, dt, Dfinal, i); });
 }
 
@@ -3578,7 +3638,7 @@ void launchFluidNeighborsDensity(const Scene &s, const Config &c, uint32_t iter,
     const Scene sp = withPositions(s, iter);
     float4 *Dk = (iter & 1u) ? s.Db : s.Da;
     const unsigned g = fluidBlocksFor(s.N);
-    const bool rebuild = s.P0 && iter > 0 && iter + fluidRebuildAhead(s.N) < s.fluidIterations;
+    const bool rebuild = s.P0 && iter > 0 && iter + kFluidRebuildAhead < s.fluidIterations;
     const uint32_t lanes = fluidLanes(s.N);
     if (s.sup && !walkCells && lanes > 1u) {
         if (s.fluidExtras) launchFluidWide<true, kFluidLanes>(sp, c, iter, Dk, rebuild, st);
@@ -3597,8 +3657,8 @@ void launchFluidNeighborsDensity(const Scene &s, const Config &c, uint32_t iter,
             else launchPdl(k_fluidNeighborsDensity<3u, false>, g, kFluidThreads, st, sp, c, true, iter, Dk);
         }
         if (rebuild) {
-            if (s.fluidExtras) launchPdl(k_fluidNeighborsDensity<4u, true>, g, kFluidThreads, st, sp, c, true, iter, Dk);
-            else launchPdl(k_fluidNeighborsDensity<4u, false>, g, kFluidThreads, st, sp, c, true, iter, Dk);
+            if (s.fluidExtras) launchPdl(k_fluidFilterAnew<true>, g, kFluidThreads, st, sp, c, iter, Dk);
+            else launchPdl(k_fluidFilterAnew<false>, g, kFluidThreads, st, sp, c, iter, Dk);
         } else {
             if (s.fluidExtras) launchPdl(k_fluidNeighborsDensity<2u, true>, g, kFluidThreads, st, sp, c, true, iter, Dk);
             else launchPdl(k_fluidNeighborsDensity<2u, false>, g, kFluidThreads, st, sp, c, true, iter, Dk);

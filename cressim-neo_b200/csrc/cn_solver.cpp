@@ -364,7 +364,9 @@ void layout(cn_solver *sv, cn::Arena &a, const cn_world_soa &w, const cn::Incide
         s.runLenSorted = a.take<uint32_t>(N); s.runCompStart = a.take<uint32_t>(N);
         s.runComp = a.take<uint32_t>(N); s.runPos = a.take<uint32_t>(N);
         s.cvals = a.take<uint32_t>(N); s.cCell = a.take<int4>(N); s.cRun = a.take<uint32_t>(N);
-        s.fluidMaxDelta = a.take<uint32_t>(64);
+        s.fluidMaxDelta = a.take<uint32_t>(192);
+        s.fluidBuilt = s.fluidMaxDelta ? s.fluidMaxDelta + 64 : nullptr;
+        s.fluidOvertaken = s.fluidMaxDelta ? s.fluidMaxDelta + 128 : nullptr;
         s.fluidIterations = sv->fluidIt;
         s.fluidMinRadius = a.take<float>(1);
         // Superset lists (k_fluidNeighborsDensity modes 1 and 2).  Without particle-particle
@@ -374,7 +376,7 @@ void layout(cn_solver *sv, cn::Arena &a, const cn_world_soa &w, const cn::Incide
         s.sup = a.take<uint32_t>(size_t(N) * s.supCap);
         s.supCount = a.take<uint32_t>(N);
         if (!sv->fluidXMoves) s.Pb = a.take<float4>(N);
-        if (sv->fluidXMoves || sv->fluidIt > 1u + cn::fluidRebuildAhead(N)) s.P0 = a.take<float4>(N);
+        if (sv->fluidXMoves || sv->fluidIt > 1u + cn::kFluidRebuildAhead) s.P0 = a.take<float4>(N);
         s.maxNbr = sv->desc.max_fluid_neighborhood;
         s.nbr = a.take<uint32_t>(std::max<size_t>(size_t(N) * s.maxNbr, 1));
         s.nbrCount = a.take<uint32_t>(N);
@@ -563,7 +565,7 @@ void enqueueFrame(cn_solver *sv, float frameDt, cudaStream_t st)
         if (s.SD) cudaMemsetAsync(s.distLambda, 0, sizeof(float) * s.SD, st);
         if (s.S) cudaMemsetAsync(s.segLambda, 0, sizeof(float4) * s.S, st);
         if (s.J) cudaMemsetAsync(s.jointLambda, 0, sizeof(float4) * s.J, st);
-        if (s.fluidMaxDelta) cudaMemsetAsync(s.fluidMaxDelta, 0, sizeof(uint32_t) * 64, st);
+        if (s.fluidMaxDelta) cudaMemsetAsync(s.fluidMaxDelta, 0, sizeof(uint32_t) * 128, st);
         if (s.hasDynamic) { // clearRigidCorrections (physics_rigid_clear_corrections.cs.hlsl)
             cudaMemsetAsync(s.bodyTransCorr, 0, sizeof(float4) * s.B, st);
             cudaMemsetAsync(s.bodyRotCorr, 0, sizeof(float4) * s.B, st);
