@@ -984,20 +984,25 @@ __device__ __forceinline__ bool neighborAllowed(const Scene &s, uint32_t tag, ui
     return om.x == m.x && (m.w & om.z) != 0u && (om.w & m.z) != 0u;
 }
 
-// Whether an iteration builds the superset lists anew: all of the scene's or none (fluids of several
-// smoothing radii have several bounds).  A list holds while its particle's candidates have moved less than
-// the margin since it was recorded, and their moves are measured from the positions of their own build.
-// Built anew where the moves are over the bound.  An iteration whose lists did not last through the next two
-// (noteSuperset) leaves it, in the substeps that follow, until the move since the last iteration is below
-// the bound for two: a fluid that outruns its lists every time only pays for recording them (4 iterations,
-// late frames of a 262K-particle gas 2,400 us a frame without, 2,530 with, a pressed block of 110K 5,050 and 5,560).
+// Whether an iteration's superset lists are due: all of the scene's or none (fluids of several smoothing radii
+// have several bounds).  A list holds while its particle's candidates have moved less than the margin since
+// it was recorded, and their moves are measured from the positions of their own build.
+__device__ __forceinline__ float supersetBound(const Scene &s) { return 0.99f * s.supMargin * __ldg(s.fluidMinRadius); }
+__device__ __forceinline__ bool supersetsDue(const Scene &s, uint32_t iter)
+{
+    return !(2.0f * __uint_as_float(s.fluidMaxDelta[iter]) < supersetBound(s));
+}
+// Whether they are built anew.  An iteration whose lists did not last through the next one (noteSuperset)
+// leaves it, in the substeps that follow, until the move since the last iteration is below the bound: a
+// fluid that outruns its lists every time only pays for recording them (4 iterations, late frames of a
+// 262K-particle gas 2,400 us a frame without, 2,530 with, a pressed block of 110K 5,050 and 5,560).
 __device__ __forceinline__ bool supersetsAnew(const Scene &s, uint32_t iter)
 {
-    const float moved = __uint_as_float(s.fluidMaxDelta[iter]), bound = 0.99f * s.supMargin * __ldg(s.fluidMinRadius);
-    if (2.0f * moved < bound) return false;
+    if (!supersetsDue(s, iter)) return false;
     if (s.fluidOvertaken[iter] == 0u) return true;
     const bool fresh = iter == 1u || s.fluidBuilt[iter - 1u] != 0u;
-    return (fresh ? moved : moved - __uint_as_float(s.fluidMaxDelta[iter - 1u])) < bound;
+    const float moved = __uint_as_float(s.fluidMaxDelta[iter]);
+    return (fresh ? moved : moved - __uint_as_float(s.fluidMaxDelta[iter - 1u])) < supersetBound(s);
 }
 __device__ __forceinline__ void supersetBuilt(const Scene &s, uint32_t iter)
 {
@@ -1005,13 +1010,11 @@ __device__ __forceinline__ void supersetBuilt(const Scene &s, uint32_t iter)
     s.fluidBuilt[0] = 1u;
 }
 
-// After a substep's iterations: whether the lists that iteration k built lasted through the next two.
+// After a substep's iterations: whether the lists that iteration k built lasted through the next one.
 __device__ __forceinline__ void noteSuperset(const Scene &s, uint32_t k)
 {
-    if (k == 0u || k + kFluidRebuildAhead >= s.fluidIterations || k + kFluidRebuildAhead >= kMaxTrackedIterations || s.fluidBuilt[k] == 0u) return;
-    const float bound = 0.99f * s.supMargin * __ldg(s.fluidMinRadius);
-    const float moved = fmaxf(__uint_as_float(s.fluidMaxDelta[k + 1u]), __uint_as_float(s.fluidMaxDelta[k + kFluidRebuildAhead]));
-    s.fluidOvertaken[k] = s.fluidBuilt[k + 1u] == 0u && 2.0f * moved < bound ? 0u : 1u;
+    if (k == 0u || k + 1u >= s.fluidIterations || k + 1u >= kMaxTrackedIterations || s.fluidBuilt[k] == 0u) return;
+    s.fluidOvertaken[k] = supersetsDue(s, k + 1u) ? 1u : 0u;
 }
 
 // Neighbour list + density constraint.
@@ -1527,7 +1530,8 @@ __global__ void __launch_bounds__(kFluidThreads, (kExtras ? 4 : 5) * (256 / kFlu
 // evaluated side by side; the sums and the list positions then run over the lanes in list order, so
 // lists and sums are the ones of the kernels above.  A thread's serial chain (a gather, a square root and
 // two divisions per neighbour, some thousand cycles) is what bounds a small scene.
-// mode 2, 3: as k_fluidNeighborsDensity; mode 4: as k_fluidFilterAnew, in one walk for both lists.
+// mode 2, 3: as k_fluidNeighborsDensity; mode 4: as k_fluidFilterAnew, in one walk
+// for both lists, wherever they are due (the lanes record beside the test, at next to no cost).
 template <uint32_t kLanes> struct LaneGroup {
     uint32_t lane, mask, shift;
     __device__ __forceinline__ LaneGroup()
@@ -1619,7 +1623,7 @@ __global__ void __launch_bounds__(kFluidThreads) k_fluidNeighborsWide(Scene s, C
     if (mode != 3u) {
         const float maxDelta = __uint_as_float(s.fluidMaxDelta[iter < kMaxTrackedIterations ? iter : 0u]);
         const bool holds = iter < kMaxTrackedIterations && 2.0f * maxDelta < 0.99f * s.supMargin * h;
-        rebuild = mode == 4u && iter + 1u < kMaxTrackedIterations && supersetsAnew(s, iter);
+        rebuild = mode == 4u && iter + 1u < kMaxTrackedIterations && supersetsDue(s, iter);
         useSuperset = holds && !rebuild && s.supCount[slot] <= s.supCap;
     }
     if (useSuperset) {
