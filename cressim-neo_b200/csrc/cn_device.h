@@ -332,6 +332,7 @@ struct Scene {
     // lists it built last did not last (kept over the substeps: it decides what is tried, not what results)
     uint32_t *fluidBuilt = nullptr, *fluidOvertaken = nullptr;
     uint32_t fluidIterations = 0;     // of a substep
+    uint32_t fluidCount = 0;          // fluid particles
     const float *fluidMinRadius = nullptr; // least smoothing radius of the fluid materials
     float4 *fluidVort = nullptr;      // curl xyz + magnitude per sorted slot (vorticity confinement)
 

@@ -3600,11 +3600,14 @@ void launchParticleCandidates(const Scene &s, uint32_t *scanTmp, size_t, cudaStr
 // iterations (true), or one walk that also builds the list and the density (false).
 constexpr bool kSplitSupersetBuild = true;
 
-// Lanes per particle of the fluid kernels: eight where a thread per particle fills less than a tenth of the
-// chip's threads.  Measured per frame of 2 substeps x 4 iterations, one lane against eight: 3,072 particles
-// 725 -> 463 us, 16,250 811 -> 603, 32,768 815 -> 767, 63,960 880 -> 1,140.
+// Lanes per particle of the fluid kernels: eight where the fluid's particles alone fill little of the chip,
+// whatever else is in the world (its other slots return at once).  Per frame of 2 substeps x 4 iterations, one
+// lane against eight: a block at rest of 8,000 particles 729 -> 506 us, of 21,952 757 -> 618, of 27,000 757 ->
+// 640, of 32,768 771 -> 693; but fluids that walk their cells gain less (the lanes share short rows): a gas of
+// 21,952 1,055 -> 1,027, of 27,000 1,077 -> 1,175, a splash of 32,768 (3 iterations) 856 -> 1,018.  A fluid of
+// 20,000 beside 24,000 particles of tissue and cloth 3,905 -> 3,600, beside 360,000 10,310 -> 10,270.
 constexpr uint32_t kFluidLanes = 8u;
-inline uint32_t fluidLanes(uint32_t n) { return n <= 32768u ? kFluidLanes : 1u; }
+inline uint32_t fluidLanes(const Scene &s) { return s.fluidCount <= 22528u && s.N <= 524288u ? kFluidLanes : 1u; }
 inline unsigned fluidWideBlocks(size_t n, uint32_t lanes) { return fluidBlocksFor(n * lanes); }
 
 template <bool kExtras, uint32_t kLanes>
@@ -3643,7 +3646,7 @@ void launchFluidNeighborsDensity(const Scene &s, const Config &c, uint32_t iter,
     float4 *Dk = (iter & 1u) ? s.Db : s.Da;
     const unsigned g = fluidBlocksFor(s.N);
     const bool rebuild = s.P0 && iter > 0 && iter + kFluidRebuildAhead < s.fluidIterations;
-    const uint32_t lanes = fluidLanes(s.N);
+    const uint32_t lanes = fluidLanes(s);
     if (s.sup && !walkCells && lanes > 1u) {
         if (s.fluidExtras) launchFluidWide<true, kFluidLanes>(sp, c, iter, Dk, rebuild, st);
         else launchFluidWide<false, kFluidLanes>(sp, c, iter, Dk, rebuild, st);
@@ -3677,7 +3680,7 @@ void launchFluidDeltaApplyClamp(const Scene &s, uint32_t iter, float dt, const C
     const float4 *Dcur = (iter & 1u) ? s.Db : s.Da;
     float4 *Dnext = (iter & 1u) ? s.Da : s.Db;
     float4 *Pnext = s.Pb ? ((iter & 1u) ? s.P : s.Pb) : nullptr;
-    const uint32_t lanes = fluidLanes(s.N);
+    const uint32_t lanes = fluidLanes(s);
     if (lanes > 1u) {
         const Scene sp = withPositions(s, iter);
         const unsigned g = fluidWideBlocks(s.N, lanes);

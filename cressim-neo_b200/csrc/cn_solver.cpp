@@ -368,6 +368,7 @@ void layout(cn_solver *sv, cn::Arena &a, const cn_world_soa &w, const cn::Incide
         s.fluidBuilt = s.fluidMaxDelta ? s.fluidMaxDelta + 64 : nullptr;
         s.fluidOvertaken = s.fluidMaxDelta ? s.fluidMaxDelta + 128 : nullptr;
         s.fluidIterations = sv->fluidIt;
+        s.fluidCount = uint32_t(std::count(w.kinds, w.kinds + N, uint32_t(CN_PARTICLE_FLUID)));
         s.fluidMinRadius = a.take<float>(1);
         // Superset lists (k_fluidNeighborsDensity modes 1 and 2).  Without particle-particle
         // contacts fluid x is fixed over the iterations and the positions are double-buffered;
