@@ -93,6 +93,7 @@ struct cn_solver {
     // Tiled soft iterations (gather schedule): the tile lists, and whether the particle-rigid
     // contacts run in the second stage
     cn::TileBuild tileBuild;
+    std::vector<char> tileStage; // kept while its upload runs
     cn::TileSet tiles{};
     bool tileContacts = false;
     float fluidMinRadius = 0.0f; // of Scene::fluidMinRadius, kept while its upload runs
@@ -213,6 +214,7 @@ void layout(cn_solver *sv, cn::Arena &a, const cn_world_soa &w, const cn::Incide
         t = cn::TileSet{};
         if (tb.ok) {
             t.tiles = uint32_t(tb.heads.size());
+            // what is uploaded side by side (uploadTiles), then the rest
             t.heads = a.take<cn::TileHead>(tb.heads.size());
             t.own = a.take<uint32_t>(tb.own.size());
             t.halo = a.take<uint32_t>(tb.halo.size());
@@ -221,11 +223,13 @@ void layout(cn_solver *sv, cn::Arena &a, const cn_world_soa &w, const cn::Incide
                 t.smem[f] = tb.smem[f];
                 t.rec[f] = a.take<uint32_t>(tb.rec[f].size());
                 t.id[f] = a.take<uint32_t>(tb.id[f].size());
-                t.ra[f] = a.take<float2>(tb.id[f].size());
-                t.lambda[f] = a.take<float>(tb.id[f].size());
             }
             t.edges = a.take<uint2>(tb.edges.size());
             t.elems = a.take<uint4>(tb.elems.size());
+            for (int f = 0; f < 2; ++f) {
+                t.ra[f] = a.take<float2>(tb.id[f].size());
+                t.lambda[f] = a.take<float>(tb.id[f].size());
+            }
             t.xB = a.take<float4>(N);
             for (const cn::TileHead &h : tb.heads) t.tetTiles += h.bends ? 0u : 1u;
         }
@@ -466,6 +470,37 @@ cn_status uploadSurfaceRender(cn_solver *sv, const cn_world_soa &w, cudaStream_t
     CN_CUDA(up(s.surfChunkRange, ranges.data(), ranges.size(), st));
     CN_CUDA(cudaStreamSynchronize(st)); // the host tables above go out of scope
     return CN_OK;
+}
+
+// The tile lists: small ones in one transfer (nine short ones took a tenth of a small scene's sync).
+cudaError_t uploadTiles(cn_solver *sv, cudaStream_t st)
+{
+    const cn::TileBuild &tb = sv->tileBuild;
+    const cn::TileSet &t = sv->tiles;
+    if (!t.tiles) return cudaSuccess;
+    struct Part {
+        const void *to, *from;
+        size_t bytes;
+    };
+    auto part = [](const auto *to, const auto &from) { return Part{to, from.data(), from.size() * sizeof(from[0])}; };
+    const Part parts[] = {part(t.heads, tb.heads),   part(t.own, tb.own),       part(t.halo, tb.halo),
+                          part(t.rec[0], tb.rec[0]), part(t.rec[1], tb.rec[1]), part(t.id[0], tb.id[0]),
+                          part(t.id[1], tb.id[1]),   part(t.edges, tb.edges),   part(t.elems, tb.elems)};
+    const char *base = reinterpret_cast<const char *>(t.heads);
+    size_t end = 0;
+    for (const Part &p : parts)
+        if (p.bytes) end = std::max(end, size_t(static_cast<const char *>(p.to) - base) + p.bytes);
+    if (end <= (size_t(256) << 10)) {
+        sv->tileStage.resize(end);
+        for (const Part &p : parts)
+            if (p.bytes) std::memcpy(sv->tileStage.data() + (static_cast<const char *>(p.to) - base), p.from, p.bytes);
+        return up(base, sv->tileStage.data(), end, st);
+    }
+    for (const Part &p : parts) {
+        const cudaError_t e = up(static_cast<const char *>(p.to), p.from, p.bytes, st);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 // The fluid materials and the least of their smoothing radii, as the kernels read a radius.
@@ -794,12 +829,7 @@ CN_API void cn_solver_destroy(cn_solver *sv)
 static uint64_t topologyHash(const cn_world_soa &w)
 {
     uint64_t h = 1469598103934665603ull;
-    auto mix = [&](uint32_t v) {
-        for (int k = 0; k < 4; ++k) {
-            h ^= (v >> (8 * k)) & 0xffu;
-            h *= 1099511628211ull;
-        }
-    };
+    auto mix = [&](uint32_t v) { h = (h ^ v) * 1099511628211ull; }; // a word at a time: the chain is what it costs
     for (uint32_t c = 0; c < w.edge_count; ++c) { mix(w.edges[c].particle_a); mix(w.edges[c].particle_b); }
     for (uint32_t c = 0; c < w.bend_count; ++c) { mix(w.bends[c].particle0); mix(w.bends[c].particle1); mix(w.bends[c].particle2); }
     for (uint32_t c = 0; c < w.dihedral_count; ++c) {
@@ -1053,33 +1083,40 @@ CN_API cn_status cn_solver_sync_world(cn_solver *sv, const cn_world_soa *w)
     // More colliders than the boundary mask holds: per-particle candidate lists over a collider LBVH
     sv->fluidBoundaryLists = anyFluid && order.size() > cn::kMaxBoundaryColliders;
 
-    // Incidence tables.
-    const cn::Incidence edgeI = cn::buildIncidence(N, w->edge_count, 2, [&](uint32_t c, uint32_t k) {
-        return k == 0 ? w->edges[c].particle_a : w->edges[c].particle_b;
-    });
-    const uint32_t nb = w->bend_count;
-    const cn::Incidence bendI = cn::buildIncidence(N, nb + w->dihedral_count, 4, [&](uint32_t c, uint32_t k) -> uint32_t {
-        if (c < nb) {
-            if (k == 3) return 0xffffffffu;
-            const cn_soft_bend &b = w->bends[c];
-            return k == 0 ? b.particle0 : (k == 1 ? b.particle1 : b.particle2);
-        }
-        const cn_cloth_dihedral &h = w->dihedrals[c - nb];
-        const uint32_t p[4] = {h.edge_particle0, h.edge_particle1, h.opposite_particle0, h.opposite_particle1};
-        return p[k];
-    });
-    const cn::Incidence tetI = cn::buildIncidence(N, w->tet_count, 4, [&](uint32_t c, uint32_t k) {
-        return w->tets[c].particle_indices[k];
-    });
-    const cn::Incidence segI = cn::buildIncidence(N, w->strand_segment_count, 2, [&](uint32_t c, uint32_t k) {
-        return k == 0 ? w->strand_segments[c].particle_a : w->strand_segments[c].particle_b;
-    });
-    const uint32_t S = w->strand_segment_count;
-    const cn::Incidence jointI = cn::buildIncidence(S, w->strand_joint_count, 2, [&](uint32_t c, uint32_t k) -> uint32_t {
-        const cn_strand_joint &j = w->strand_joints[c];
-        if (j.segment_a >= S || j.segment_b >= S) return 0xffffffffu;
-        return k == 0 ? j.segment_a : j.segment_b;
-    });
+    // Incidence tables, side by side where they take longer than starting the threads.
+    const uint32_t nb = w->bend_count, S = w->strand_segment_count;
+    cn::Incidence edgeI, bendI, tetI, segI, jointI;
+    const auto tables = [&](uint32_t task) {
+        if (task == 0u)
+            tetI = cn::buildIncidence(N, w->tet_count, 4, [&](uint32_t c, uint32_t k) {
+                return w->tets[c].particle_indices[k];
+            });
+        if (task == 1u)
+            edgeI = cn::buildIncidence(N, w->edge_count, 2, [&](uint32_t c, uint32_t k) {
+                return k == 0 ? w->edges[c].particle_a : w->edges[c].particle_b;
+            });
+        if (task != 2u) return;
+        bendI = cn::buildIncidence(N, nb + w->dihedral_count, 4, [&](uint32_t c, uint32_t k) -> uint32_t {
+            if (c < nb) {
+                if (k == 3) return 0xffffffffu;
+                const cn_soft_bend &b = w->bends[c];
+                return k == 0 ? b.particle0 : (k == 1 ? b.particle1 : b.particle2);
+            }
+            const cn_cloth_dihedral &h = w->dihedrals[c - nb];
+            const uint32_t p[4] = {h.edge_particle0, h.edge_particle1, h.opposite_particle0, h.opposite_particle1};
+            return p[k];
+        });
+        segI = cn::buildIncidence(N, w->strand_segment_count, 2, [&](uint32_t c, uint32_t k) {
+            return k == 0 ? w->strand_segments[c].particle_a : w->strand_segments[c].particle_b;
+        });
+        jointI = cn::buildIncidence(S, w->strand_joint_count, 2, [&](uint32_t c, uint32_t k) -> uint32_t {
+            const cn_strand_joint &j = w->strand_joints[c];
+            if (j.segment_a >= S || j.segment_b >= S) return 0xffffffffu;
+            return k == 0 ? j.segment_a : j.segment_b;
+        });
+    };
+    if (uint64_t(w->edge_count) + w->tet_count + nb + w->dihedral_count > 32768u) cn::runParallel(3u, tables);
+    else for (uint32_t task = 0; task < 3u; ++task) tables(task);
 
     // XPBD schedule: the coloured schedules colour every family (elements: particles; segments
     // for the joints, whose corrections move orientations)
@@ -1227,19 +1264,7 @@ CN_API cn_status cn_solver_sync_world(cn_solver *sv, const cn_world_soa *w)
         CN_CUDA(up(const_cast<uint32_t *>(sv->plan.devStarts[f]), col.starts.data(), col.starts.size(), st));
     }
     CN_CUDA(uploadColourOrdered(sv, *w, st));
-    if (sv->tiles.tiles) {
-        const cn::TileBuild &tb = sv->tileBuild;
-        const cn::TileSet &t = sv->tiles;
-        CN_CUDA(up(t.heads, tb.heads.data(), tb.heads.size(), st));
-        CN_CUDA(up(t.own, tb.own.data(), tb.own.size(), st));
-        CN_CUDA(up(t.halo, tb.halo.data(), tb.halo.size(), st));
-        for (int f = 0; f < 2; ++f) {
-            CN_CUDA(up(t.rec[f], tb.rec[f].data(), tb.rec[f].size(), st));
-            CN_CUDA(up(t.id[f], tb.id[f].data(), tb.id[f].size(), st));
-        }
-        CN_CUDA(up(t.edges, tb.edges.data(), tb.edges.size(), st));
-        CN_CUDA(up(t.elems, tb.elems.data(), tb.elems.size(), st));
-    }
+    CN_CUDA(uploadTiles(sv, st));
     CN_CUDA(up(s.bodyPos, w->body_positions_inv_mass, s.B, st));
     CN_CUDA(up(s.bodyRot, w->body_orientations, s.B, st));
     CN_CUDA(up(s.bodyLin, w->body_linear_velocities, s.B, st));
