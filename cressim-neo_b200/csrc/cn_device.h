@@ -535,7 +535,7 @@ void launchTileEdges(const Scene &s, const TileSet &t, const Config &c, uint32_t
 void launchTileTets(const Scene &s, const TileSet &t, const Config &c, uint32_t flags, bool contacts, cudaStream_t st);
 void launchTileBends(const Scene &s, const TileSet &t, const Config &c, uint32_t flags, bool contacts, cudaStream_t st);
 // Every iteration of a substep of a coloured schedule in one CTA, the positions in its shared memory.
-bool residentColourFits(const Scene &s, const XpbdPlan &plan);
+bool residentColourFits(const Scene &s, const XpbdPlan &plan, bool rigid);
 void launchResidentColour(const Scene &s, const Config &c, float dt, const XpbdPlan &plan, uint32_t iterations,
                           uint32_t softIterations, uint32_t contactIterations, bool rigid, cudaStream_t st);
 // Allows the kernels `bytes` of dynamic shared memory per CTA; false when the device has less.

@@ -4347,9 +4347,29 @@ static size_t residentColourBytes(const Scene &s, const XpbdPlan &plan)
            size_t(s.T) * sizeof(ColourTet) + (size_t(plan.colours[kFamEdges]) + plan.colours[kFamTets] + 2u) * sizeof(uint32_t);
 }
 
-bool residentColourFits(const Scene &s, const XpbdPlan &plan)
+// One CTA runs at one SM's throughput, launches at the chip's with ~2.4 us each: per iteration, in ns, the
+// work against the launches.  Measured in frames of 2 substeps x 10 iterations, launches against one CTA: a
+// block of 1,000 particles (56 colours) 3,370 -> 1,120 us; a cloth (20 colours) of 784 1,370 -> 930, of 1,024
+// 1,360 -> 1,170, of 1,296 1,400 -> 1,550, of 2,304 1,450 -> 2,540; a strand (6 colours) of 600 544 -> 390, of
+// 1,000 540 -> 546, of 5,000 560 -> 2,160; a body of edges alone of 2,000 (13 colours) 900 -> 520, of 5,000
+// (5) 430 -> 495.
+static bool residentColourPays(const Scene &s, const XpbdPlan &plan, bool rigid)
 {
-    if (s.N > 0xffffu || residentColourBytes(s, plan) > kResidentSmemCap) return false;
+    const uint64_t sizes[kFamilies] = {s.E, s.S, uint64_t(s.Bn) + s.D, s.J, s.SD, s.T};
+    constexpr double kConstraint[kFamilies] = {1.5, 3.0, 10.0, 3.0, 3.0, 3.0}; // edges and tets from shared memory
+    constexpr double kColour = 600.0, kContact = 4.0, kLaunch = 2400.0;
+    double work = rigid ? kContact * s.N : 0.0, launches = rigid ? 1.0 : 0.0;
+    for (uint32_t f = 0; f < kFamilies; ++f) {
+        if (sizes[f] == 0u) continue;
+        work += kConstraint[f] * double(sizes[f]) + kColour * plan.colours[f];
+        launches += plan.colours[f];
+    }
+    return work <= kLaunch * launches;
+}
+
+bool residentColourFits(const Scene &s, const XpbdPlan &plan, bool rigid)
+{
+    if (s.N > 0xffffu || residentColourBytes(s, plan) > kResidentSmemCap || !residentColourPays(s, plan, rigid)) return false;
     for (const void *f : {reinterpret_cast<const void *>(&k_residentColour<true>), reinterpret_cast<const void *>(&k_residentColour<false>)})
         if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kResidentSmemCap)) != cudaSuccess) {
             cudaGetLastError();

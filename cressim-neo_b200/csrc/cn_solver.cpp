@@ -1312,7 +1312,7 @@ CN_API cn_status cn_solver_sync_world(cn_solver *sv, const cn_world_soa *w)
                          !sv->hasDynamic && !sv->rigidRigid && nProxy == 0 &&
                          (s.E || s.Bn || s.D || s.T || s.S || s.J || s.SD) &&
                          constraintIndicesValid(*w) &&
-                         cn::residentColourFits(s, sv->plan);
+                         cn::residentColourFits(s, sv->plan, sv->rigidPossible);
     // Concurrent branches (per-phase gather schedule): the strand families beside the others, the
     // cloth bends beside the tets once the edges are applied, and the fluid chain beside the soft
     // families, whenever the particle windows they write are disjoint.

@@ -116,6 +116,31 @@ def test_restitution_after_the_iterations():
     _equal(*_states(w, desc, 4))
 
 
+# a strand and a cloth on the ground within what one CTA does faster than a launch per colour, and over it; a
+# launch per colour makes 10 iterations of 6 (20) colours
+@pytest.mark.parametrize("schedule", [1, 2])
+@pytest.mark.parametrize("kind, n, resident", [("strand", 600, True), ("strand", 2000, False), ("cloth", 30, True),
+                                               ("cloth", 40, False)])
+def test_resident_colours_stop_where_launches_are_faster(schedule, kind, n, resident):
+    w = World()
+    if kind == "strand":
+        w.add_strand([(0.0, 0.02, 0.02 * k) for k in range(n)], radius=0.01, stretch_shear_compliance=1e-6, bend_compliance=1e-4,
+                     twist_compliance=1e-4, static_particles=[0])
+    else:
+        w.add_cloth_grid((n, n), (0.02 * n, 0.02 * n), position=(0.0, 0.01, 0.0), radius=0.008, structural_compliance=1e-6,
+                         bend_compliance=1e-3, static_particles=[0], friction=0.2)
+    scenes.ground(w)
+    desc = solver_desc(substeps=1, default_iterations=10, enable_blocking_readback=0)
+    desc.soft.xpbd_schedule = schedule
+    gpu, ora = Solver(desc), cn_oracle.Oracle(desc, w.soa())
+    gpu.sync_world(w)
+    gpu.step(1.0 / 60.0)
+    ora.step(1.0 / 60.0)
+    assert (gpu.graph_stats()[0] < 20) == resident
+    for g, o in zip(gpu.read_particles(), ora.read_particles()):
+        np.testing.assert_allclose(g, o, rtol=1e-5, atol=1e-5)
+
+
 @pytest.mark.parametrize("schedule", [1, 2])
 def test_resident_colours_with_a_particle_named_twice(schedule):
     w = _block((4, 4, 4), pinned=False)
