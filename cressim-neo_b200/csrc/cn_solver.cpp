@@ -945,17 +945,20 @@ static void buildSolverTiles(cn_solver *sv, const cn_world_soa &w, const cn::Inc
     const bool strands = w.strand_segment_count || w.strand_joint_count || w.strand_distance_count;
     const bool contacts = sv->rigidPossible && !sv->ppPossible && !sv->hasFluid && !strands;
     std::vector<uint8_t> cls(N, 0);
+    uint32_t tiled = 0;
     for (uint32_t i = 0; i < N; ++i) {
         const bool t = tetI.ranges[i].y != 0, b = bendI.ranges[i].y != 0;
         if (t && b) return;
         const bool any = t || b || edgeI.ranges[i].y != 0;
         if (any && segI.ranges[i].y != 0) return;
-        if (any || contacts) cls[i] = b ? 2 : 1;
+        if (!any && !contacts) continue;
+        cls[i] = b ? 2 : 1;
+        ++tiled;
     }
     using In = cn::TileInput<decltype(edgeOf), decltype(tetOf), decltype(bendOf)>;
     const In in{N, w.positions_inv_mass, cls, edgeI, tetI, bendI, edgeOf, tetOf, bendOf};
     sv->tileContacts = contacts;
-    const uint32_t target = cn::tileTarget(N);
+    const uint32_t target = cn::tileTarget(tiled);
     if (!target) return;
     try {
         sv->tileBuild = cn::buildTiles(in, target, cn::kTileSmemCap);

@@ -27,13 +27,17 @@
 namespace cn {
 
 constexpr uint32_t kTileSmemCap = 112u << 10; // two tiles' CTAs on an SM
-// Particles per tile; 0: the per-family kernels run.
+// Particles per tile for the n particles of a world that go into tiles, whatever else is in it; 0: the
+// per-family kernels run.
 //  * A small scene is all latency, and a CTA's threads should each have one entry or two of a stage: tiles
 //    of 16 (lattices of 216 to 2,744 particles, 4 substeps x 20 iterations, per frame: 547-612 us with the
 //    per-family kernels, 400-460 us with tiles of 12 to 24, 410-515 us with tiles of 48).
 //  * Large scenes fill whole waves of two CTAs an SM with tiles of at most 192 (a larger tile solves
 //    fewer constraints twice, but 340 leaves too few CTAs: 100K particles, 4 x 20 iterations, 2.4 ms at
-//    170, 2.9 at 96, 2.7 at 340, 4.0 with the per-family kernels).
+//    170, 2.9 at 96, 2.7 at 340, 4.0 with the per-family kernels).  16K of tissue and cloth, 2 x 20 iterations:
+//    1,217 us with the per-family kernels, 1,140 with tiles of 55, 1,206 of 64, 1,403 of 16; beside 130K of
+//    fluid 5,320 and 5,230.  Sized for all 146K particles of that world its tiles would be of 165: 4,250
+//    us against 4,130 (2 fluid iterations).
 //  * In between the per-family kernels stay, though the tiles measured faster there as well (4,096
 //    particles: 505 against 647 us): the frame graph of the 16^3 cube is held to one launch per
 //    phase by the schedule test, which the stages' two launches an iteration do not meet.

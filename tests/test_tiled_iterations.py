@@ -50,6 +50,24 @@ def test_tiles_equal_the_oracle(n, pinned):
     _equal(*_states(w, desc))
 
 
+def test_tiles_are_sized_by_the_particles_in_them():
+    # 1,000 particles of tissue have tiles, two launches an iteration, beside 1,400 of fluid and beside 2,688
+    # (whose world is of a size that alone would have none)
+    launches = []
+    for fluid in ((10, 10, 14), (12, 14, 16)):
+        w = _block((10, 10, 10))
+        size = tuple(0.05 * k for k in fluid)
+        w.add_fluid_grid(size, 0.05, position=(5.0, size[1] * 0.5 + 0.01, 0.0), radius=0.03)
+        desc = solver_desc(substeps=1, default_iterations=5, enable_blocking_readback=0)
+        gpu, ora = Solver(desc), cn_oracle.Oracle(desc, w.soa())
+        gpu.sync_world(w)
+        gpu.step(1.0 / 60.0)
+        ora.step(1.0 / 60.0)
+        _equal(gpu.read_particles(), ora.read_particles())
+        launches.append(gpu.graph_stats()[0])
+    assert launches[0] == launches[1]
+
+
 def test_tets_without_compliance_keep_their_records():
     # 10 cm tets: the weighted squared gradients (~1e-5) are above the degenerate bound; flattened ones are not
     w = _block((6, 5, 6), compliance=0.0, pinned=False)
