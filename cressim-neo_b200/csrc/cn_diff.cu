@@ -515,18 +515,10 @@ void copyAsync(void *dst, const void *src, size_t bytes, cudaStream_t st)
     if (bytes) cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, st);
 }
 
+// A kernel of the iterations over `threads`, launched ahead of its predecessor's end.
 template <class... P, class... A> void launchDependent(void (*k)(P...), size_t threads, cudaStream_t st, A... args)
 {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(gridOf(threads), 1, 1);
-    cfg.blockDim = dim3(kDiffThreads, 1, 1);
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k, P(args)...);
+    cn::launchPdl(k, gridOf(threads), unsigned(kDiffThreads), st, args...);
 }
 
 // One substep of the state (g.x, g.v).  With `record` every iteration writes its positions and lambdas to
