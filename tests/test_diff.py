@@ -137,6 +137,88 @@ def test_adjoint_matches_fp64_central_differences():
     assert rel < 2e-2 and cosv > 0.99, (rel, cosv)
 
 
+# one family alone: its iterations follow one another directly (edges of a mesh-free body; the tets of a block
+# whose edges are left out)
+@pytest.mark.gpu
+@pytest.mark.parametrize("family", ["edges", "tets"])
+def test_adjoint_of_one_family_matches_fp64_central_differences(family):
+    import torch
+    if family == "edges":
+        w = World()
+        w.add_soft_body_meshfree(np.random.default_rng(3).uniform(0.0, 0.5, (120, 3)), 6, position=(0.0, 0.5, 0.0), radius=0.02,
+                                 edge_compliance=1e-5)
+        soa = w.soa()
+    else:
+        w = block((5, 4, 4))
+        soa = w.soa()
+        soa.edge_count = 0
+    r = diff.Rollout(soa, substeps=6, iterations=5, substep_dt=1.0 / 480.0, checkpoint_interval=4, precision=8)
+    comp, x0, v0 = _inputs(w, torch, torch.float64)
+    if family == "edges":
+        comp = torch.ones(1, device="cuda", dtype=torch.float64)    # a buffer without entries has no address
+    rng = np.random.default_rng(7)
+    g = torch.as_tensor(rng.normal(0.0, 1.0, x0.shape), device="cuda")
+    g[:, 3] = 0
+
+    def value(c, x, v):
+        out = torch.empty_like(x)
+        r.forward(c, x, v, out)
+        return float((out * g).sum())
+
+    value(comp, x0, v0)
+    gc, gx, gv = torch.zeros_like(comp), torch.zeros_like(x0), torch.zeros_like(v0)
+    r.backward(g, None, gc, gx, gv)
+    torch.cuda.synchronize()
+    ux, uv = (torch.as_tensor(rng.normal(0.0, 1.0, x0.shape), device="cuda") * (x0[:, 3:] > 0) for _ in range(2))
+    ux[:, 3] = uv[:, 3] = 0
+    uc = torch.as_tensor(rng.normal(0.0, 1.0, comp.shape[0]), device="cuda") * comp
+    # central differences of a function of order 1 to 10: truncation eps^2, rounding 1e-15 / eps
+    for eps, grad, u, at in ((1e-6, gx, ux, 1), (1e-6, gv, uv, 2), (1e-4, gc, uc, 0)):
+        if at == 0 and family == "edges":
+            continue
+        args = [comp, x0, v0]
+        args[at] = args[at] + eps * u
+        up = value(*args)
+        args[at] = args[at] - 2 * eps * u
+        fd, an = (up - value(*args)) / (2 * eps), float((grad * u).sum())
+        assert abs(an - fd) <= 1e-5 * abs(fd) + 1e-7, (at, an, fd)
+
+
+# on a stream that is being captured the launches go into the caller's graph one by one; before the engine has its
+# own graphs, and after
+@pytest.mark.gpu
+@pytest.mark.parametrize("first", ["capture", "eager"])
+def test_captured_rollout_equals_the_eager_one(first):
+    import torch
+    w = block((6, 5, 5))
+    kw = dict(substeps=6, iterations=5, substep_dt=1.0 / 480.0, checkpoint_interval=4)
+    comp, x0, v0 = _inputs(w, torch, torch.float32)
+    g = torch.zeros_like(x0)
+    g[:, :3] = torch.as_tensor(np.random.default_rng(5).normal(0.0, 1.0, (len(x0), 3)), device="cuda", dtype=torch.float32)
+
+    def run(r, c, x, v):
+        out, gc, gx, gv = torch.empty_like(x), torch.zeros_like(c), torch.zeros_like(x), torch.zeros_like(v)
+        r.forward(c, x, v, out)
+        r.backward(g, None, gc, gx, gv)
+        return out, gc, gx, gv
+
+    r = diff.Rollout(w, **kw)
+    if first == "eager":
+        run(r, comp, x0, v0)
+    held = [t.clone() for t in (comp, x0, v0)]
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = run(r, *held)
+    for scale in (1.0, 1.5):        # replayed on other inputs in the same tensors
+        held[0].copy_(comp * scale)
+        held[2].copy_(v0 * scale)
+        graph.replay()
+        torch.cuda.synchronize()
+        for a, b in zip(got, run(diff.Rollout(w, **kw), comp * scale, x0, v0 * scale)):
+            assert torch.equal(a, b)
+
+
 @pytest.mark.gpu
 def test_checkpoint_interval_does_not_change_gradients():
     import torch
