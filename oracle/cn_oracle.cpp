@@ -3423,6 +3423,20 @@ CN_API cno_solver *cno_create(const cn_solver_desc *desc, const cn_world_soa *wo
 
 CN_API void cno_destroy(cno_solver *s) { delete s; }
 
+// The constraint records of `world` (the same constraints, other values), as an incremental update of the
+// reference's scene buffers: what the solver has kept between frames stays.
+CN_API int cno_update_constraints(cno_solver *s, const cn_world_soa *world)
+{
+    if (!s || !world || world->edge_count != s->edges.size() || world->bend_count != s->bends.size() ||
+        world->dihedral_count != s->dihedrals.size() || world->tet_count != s->tets.size())
+        return CN_ERR_INVALID_ARGUMENT;
+    copyArr(s->edges, world->edges, world->edge_count);
+    copyArr(s->bends, world->bends, world->bend_count);
+    copyArr(s->dihedrals, world->dihedrals, world->dihedral_count);
+    copyArr(s->tets, world->tets, world->tet_count);
+    return CN_OK;
+}
+
 // Switches the reference's post-update neighbour rebuild off (lists then hold the last
 // iteration's build), for comparisons with a GPU schedule that skips it.
 CN_API void cno_set_post_update_neighbors(cno_solver *s, int enable) { s->postUpdateNeighbors = enable != 0; }

@@ -37,6 +37,7 @@ def load(quotients: bool = False) -> C.CDLL:
         lib.cno_create.restype = C.c_void_p
         lib.cno_create.argtypes = [C.c_void_p, C.c_void_p]
         lib.cno_destroy.argtypes = [C.c_void_p]
+        lib.cno_update_constraints.argtypes = [C.c_void_p, C.c_void_p]
         lib.cno_step.argtypes = [C.c_void_p, C.c_float]
         lib.cno_read_particles.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]
         lib.cno_read_strand_orientations.argtypes = [C.c_void_p, C.c_void_p]
@@ -86,6 +87,11 @@ class Oracle:
 
     def set_post_update_neighbors(self, enable: bool) -> None:
         self._lib.cno_set_post_update_neighbors(self._h, int(enable))
+
+    def update_constraints(self, soa) -> None:
+        """The values of the constraint records (the same constraints as at creation)."""
+        if self._lib.cno_update_constraints(self._h, C.byref(soa)):
+            raise ValueError("oracle: other constraints")
 
     def step(self, dt: float) -> None:
         self._lib.cno_step(self._h, dt)

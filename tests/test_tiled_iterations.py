@@ -11,12 +11,11 @@ from cn_physics import Solver, World, scenes, solver_desc
 pytestmark = pytest.mark.gpu
 
 
-def _block(n, compliance=1e-6, pinned=True, seed=0):
+def _block(n, compliance=1e-6, pinned=True, seed=0, sp=0.1):
     w = World()
-    sp = 0.1
     size = tuple((k - 1.25) * sp for k in n)
     static = [x * n[1] * n[2] + z for x in range(n[0]) for z in range(n[2])] if pinned else []
-    w.add_soft_body_grid(size, sp, position=(0.0, size[1] * 0.5 + 0.04, 0.0), radius=0.04, edge_compliance=1e-5,
+    w.add_soft_body_grid(size, sp, position=(0.0, size[1] * 0.5 + 0.04, 0.0), radius=0.4 * sp, edge_compliance=1e-5,
                          volume_compliance=compliance, static_particles=static, friction=0.3)
     scenes.ground(w)
     w.soa()
@@ -26,14 +25,31 @@ def _block(n, compliance=1e-6, pinned=True, seed=0):
 
 
 def _states(w, desc, frames=2, edit=None):
+    """States of the two sides; `edit` changes the world's constraints before the second frame."""
     gpu, ora = Solver(desc), cn_oracle.Oracle(desc, w.soa())
     gpu.sync_world(w)
     for k in range(frames):
         if edit is not None and k == 1:
-            edit(gpu, ora)
+            edit()
+            gpu.update_world(w, "constraints")
+            ora.update_constraints(w.soa())
         gpu.step(1.0 / 60.0)
         ora.step(1.0 / 60.0)
     return gpu.read_particles(), ora.read_particles()
+
+
+def _launches(w, desc):
+    """Launches of one iteration, by which the path that runs is told: two on tiles (edges, then tets or bends
+    with the contacts), four by family, none in the one CTA of a coloured schedule."""
+    count = []
+    for iterations in (desc.default_iterations, desc.default_iterations + 1):
+        d = type(desc).from_buffer_copy(desc)
+        d.default_iterations = iterations
+        gpu = Solver(d)
+        gpu.sync_world(w)
+        gpu.step(1.0 / 60.0)
+        count.append(gpu.graph_stats()[0])
+    return (count[1] - count[0]) // desc.substeps
 
 
 def _equal(a, b):
@@ -41,13 +57,16 @@ def _equal(a, b):
         assert np.array_equal(np.asarray(g).view(np.uint32), np.asarray(o).view(np.uint32)), float(np.abs(g - o).max())
 
 
-# one tile; a few; the last size of the small range; the first tiled one above it; two waves' partial one
-@pytest.mark.parametrize("n", [(2, 2, 2), (5, 4, 3), (16, 12, 16), (18, 18, 19), (27, 21, 23)])
+# one tile; a few; the last size of the small range (3,072); the sizes without tiles next to it and to the first one
+# above (6,144); two waves' partial one
+@pytest.mark.parametrize("n, launches", [((2, 2, 2), 2), ((5, 4, 3), 2), ((16, 12, 16), 2), ((11, 14, 20), 4), ((17, 19, 19), 4),
+                                         ((16, 16, 24), 2), ((18, 18, 19), 2), ((27, 21, 23), 2)])
 @pytest.mark.parametrize("pinned", [True, False])
-def test_tiles_equal_the_oracle(n, pinned):
+def test_tiles_equal_the_oracle(n, launches, pinned):
     w = _block(n, pinned=pinned)
     desc = solver_desc(substeps=2, default_iterations=5, enable_blocking_readback=0)
     _equal(*_states(w, desc))
+    assert _launches(w, desc) == launches
 
 
 def test_tiles_are_sized_by_the_particles_in_them():
@@ -68,13 +87,33 @@ def test_tiles_are_sized_by_the_particles_in_them():
     assert launches[0] == launches[1]
 
 
-def test_tets_without_compliance_keep_their_records():
-    # 10 cm tets: the weighted squared gradients (~1e-5) are above the degenerate bound; flattened ones are not
-    w = _block((6, 5, 6), compliance=0.0, pinned=False)
-    x = w.positions()
-    x[x[:, 0] > 0.1, 1] *= np.float32(1e-3)
+# A tet without compliance whose weighted squared gradients are under the bound (1e-6) keeps its last corrections.
+# At 5.2 cm and a particle mass of 1 kg they are 0.8e-6 to 2.2e-6, a median of 1e-6: tets go from one side to the other
+# (records cleared after the first frame change the oracle's positions by 4 mm).
+@pytest.mark.parametrize("schedule", [0, 1, 2])
+def test_tets_without_compliance_keep_their_records(schedule):
+    w = _block((6, 5, 6), compliance=0.0, pinned=False, sp=0.052)
     desc = solver_desc(substeps=2, default_iterations=4, enable_blocking_readback=0)
+    desc.soft.xpbd_schedule = schedule
     _equal(*_states(w, desc, 3))
+    assert _launches(w, desc) == (0 if schedule else 2)
+
+
+# After a frame every tet loses its compliance, at 4 cm and 1 kg under the bound (3e-7 to 8e-7; 3e-6 of scaled
+# compliance before): they keep the corrections of the iteration before the change.  And every third edge is switched.
+@pytest.mark.parametrize("schedule", [0, 1, 2])
+def test_constraints_changed_between_frames(schedule):
+    w = _block((6, 5, 6), compliance=2e-10, pinned=False, sp=0.04)
+
+    def edit():
+        w.array("tets").view(np.float32)[:, 5] = 0.0
+        e = w.array("edges")
+        e[::3, 4] = 1 - e[::3, 4]
+
+    desc = solver_desc(substeps=2, default_iterations=4, enable_blocking_readback=0)
+    desc.soft.xpbd_schedule = schedule
+    _equal(*_states(w, desc, 3, edit))
+    assert _launches(w, desc) == (0 if schedule else 2)
 
 
 def test_disabled_edges_and_a_hub():
@@ -86,6 +125,7 @@ def test_disabled_edges_and_a_hub():
     e[:, 1][e[:, 0] == e[:, 1]] = 101
     desc = solver_desc(substeps=2, default_iterations=4, enable_blocking_readback=0, soft_internal_relaxation=0.02)
     _equal(*_states(w, desc))
+    assert _launches(w, desc) == 2
 
 
 def test_edges_alone():
@@ -95,6 +135,7 @@ def test_edges_alone():
     scenes.ground(w)
     desc = solver_desc(substeps=2, default_iterations=5, enable_blocking_readback=0)
     _equal(*_states(w, desc))
+    assert _launches(w, desc) == 2
 
 
 @pytest.mark.parametrize("resolution", [(7, 5), (90, 80)])
@@ -106,16 +147,35 @@ def test_cloth_tiles(resolution):
     desc = solver_desc(substeps=2, default_iterations=5, enable_blocking_readback=0)
     for g, o in zip(*_states(w, desc)):
         np.testing.assert_allclose(g, o, rtol=1e-5, atol=1e-5)
+    assert _launches(w, desc) == 2
+
+
+def test_edges_between_tiles_of_tets_and_of_bends():
+    # a tile holds particles with tets or particles with bends: these edges have one end in each
+    w = _block((6, 5, 6))
+    tissue = len(w.positions())
+    w.add_cloth_grid((9, 8), (0.4, 0.35), position=(0.0, 0.8, 0.0), radius=0.008, structural_compliance=1e-6, bend_compliance=1e-3,
+                     friction=0.2)
+    w.soa()
+    e = w.array("edges")
+    across = np.arange(0, len(e), 40)
+    e[across, 0], e[across, 1] = np.arange(len(across)), tissue + np.arange(len(across)) % 72
+    e.view(np.float32)[across, 2] = 0.5
+    desc = solver_desc(substeps=2, default_iterations=5, enable_blocking_readback=0)
+    for g, o in zip(*_states(w, desc)):
+        np.testing.assert_allclose(g, o, rtol=1e-5, atol=1e-5)
+    assert _launches(w, desc) == 8      # edges, tets, bends (seven by family); five of the contacts between the two bodies
 
 
 # within one CTA; colours larger than its threads; past its shared memory (a launch per colour)
 @pytest.mark.parametrize("schedule", [1, 2])
-@pytest.mark.parametrize("n, pinned", [((3, 3, 3), False), ((10, 9, 11), True), ((13, 13, 13), True)])
-def test_resident_colours_equal_the_oracle(schedule, n, pinned):
+@pytest.mark.parametrize("n, pinned, resident", [((3, 3, 3), False, True), ((10, 9, 11), True, True), ((13, 13, 13), True, False)])
+def test_resident_colours_equal_the_oracle(schedule, n, pinned, resident):
     w = _block(n, pinned=pinned)
     desc = solver_desc(substeps=2, default_iterations=3, enable_blocking_readback=0)
     desc.soft.xpbd_schedule = schedule
     _equal(*_states(w, desc))
+    assert (_launches(w, desc) == 0) == resident
 
 
 def test_restitution_after_the_iterations():
@@ -134,8 +194,7 @@ def test_restitution_after_the_iterations():
     _equal(*_states(w, desc, 4))
 
 
-# a strand and a cloth on the ground within what one CTA does faster than a launch per colour, and over it; a
-# launch per colour makes 10 iterations of 6 (20) colours
+# a strand and a cloth on the ground within what one CTA does faster than a launch per colour, and over it
 @pytest.mark.parametrize("schedule", [1, 2])
 @pytest.mark.parametrize("kind, n, resident", [("strand", 600, True), ("strand", 2000, False), ("cloth", 30, True),
                                                ("cloth", 40, False)])
@@ -150,13 +209,9 @@ def test_resident_colours_stop_where_launches_are_faster(schedule, kind, n, resi
     scenes.ground(w)
     desc = solver_desc(substeps=1, default_iterations=10, enable_blocking_readback=0)
     desc.soft.xpbd_schedule = schedule
-    gpu, ora = Solver(desc), cn_oracle.Oracle(desc, w.soa())
-    gpu.sync_world(w)
-    gpu.step(1.0 / 60.0)
-    ora.step(1.0 / 60.0)
-    assert (gpu.graph_stats()[0] < 20) == resident
-    for g, o in zip(gpu.read_particles(), ora.read_particles()):
+    for g, o in zip(*_states(w, desc, 1)):
         np.testing.assert_allclose(g, o, rtol=1e-5, atol=1e-5)
+    assert (_launches(w, desc) == 0) == resident
 
 
 @pytest.mark.parametrize("schedule", [1, 2])
