@@ -459,11 +459,15 @@ void launchParticleCandidates(const Scene &s, uint32_t *scanTmp, size_t scanTmpB
 void launchFluidIteration(const Scene &s, uint32_t iter, float dt, const Config &c, bool writeDebug,
                           cudaStream_t st);
 void launchFluidGather(const Scene &s, uint32_t iter, cudaStream_t st);
-// Iterations that have to follow for the superset lists to be built anew where the moves are over their bound:
-// recording them costs about half a walk of the cells, which two filters in place of walks repay (4
-// iterations: a 480K-particle splash 3,490 -> 3,220 us a frame, 1M particles 6,940 -> 6,610; a fluid at rest
-// the same).
-constexpr uint32_t kFluidRebuildAhead = 2u;
+// Fluids of up to so many particles find their neighbours with eight lanes each (fluidLanes); larger ones fill
+// the chip.
+constexpr uint32_t kFluidWide = 22528u;
+// Iterations that have to follow for the superset lists of n fluid particles to be built anew where the moves
+// are over their bound: recording them costs about half a walk of the cells, which two filters in place of
+// walks repay where all of a fluid is stirred (4 iterations, 480K particles 3,490 -> 3,220 us a frame, 120K 1,490 ->
+// 1,310) and just not where a few of its particles are over the bound (1M particles 5,545 -> 5,660, 610K 3,530 ->
+// 3,590, 120K 1,205 -> 1,183): with two for the smaller, four for the larger.
+inline uint32_t fluidRebuildAhead(uint32_t n) { return n < 262144u ? 2u : 4u; }
 // False when the positions are double-buffered: the gather then runs at the first iteration only.
 bool fluidGatherEachIteration(const Scene &s);
 // walkCells: every iteration walks the 27 cells (no superset lists).

@@ -1245,7 +1245,7 @@ __global__ void __launch_bounds__(kFluidThreads, (kExtras ? 4 : 5) * (256 / kFlu
 
 // The pair term, the boundary part and the apply of the position delta as functions, for k_fluidDeltaWide.
 // k_fluidDeltaApplyClamp below holds the same expressions in its body: through these its register allocation
-// comes out 1 % slower at 1M particles.
+// comes out 0.8 % slower at 1M particles.  The tests hold both to the oracle, bit for bit.
 // What a particle brings to its pair terms.
 struct FluidSelf {
     f3 sp, sdl, sn;
@@ -3601,13 +3601,14 @@ void launchParticleCandidates(const Scene &s, uint32_t *scanTmp, size_t, cudaStr
 constexpr bool kSplitSupersetBuild = true;
 
 // Lanes per particle of the fluid kernels: eight where the fluid's particles alone fill little of the chip,
-// whatever else is in the world (its other slots return at once).  Per frame of 2 substeps x 4 iterations, one
-// lane against eight: a block at rest of 8,000 particles 729 -> 506 us, of 21,952 757 -> 618, of 27,000 757 ->
-// 640, of 32,768 771 -> 693; but fluids that walk their cells gain less (the lanes share short rows): a gas of
-// 21,952 1,055 -> 1,027, of 27,000 1,077 -> 1,175, a splash of 32,768 (3 iterations) 856 -> 1,018.  A fluid of
-// 20,000 beside 24,000 particles of tissue and cloth 3,905 -> 3,600, beside 360,000 10,310 -> 10,270.
+// whatever else is in the world (its other slots return at once).  Per frame of 2 substeps, one lane against
+// eight.  Neighbour kernels: a block at rest of 17,576 particles, 4 iterations, 731 -> 638 us, of 27,000 763 -> 729; but
+// fluids that walk their cells gain less (the lanes share short rows): a splash of 21,952, 3 iterations, 1,210 -> 1,020,
+// of 27,000 a gas 941 -> 1,064, of 32,768 859 -> 1,079.  Delta kernel: a block at rest of 17,576 731 -> 643, of
+// 32,768 772 -> 738, a gas of 32,768 1,111 -> 1,036, of 46,656 and 20 iterations at rest 2,154 -> 2,209.
 constexpr uint32_t kFluidLanes = 8u;
-inline uint32_t fluidLanes(const Scene &s) { return s.fluidCount <= 22528u && s.N <= 524288u ? kFluidLanes : 1u; }
+inline uint32_t fluidLanes(const Scene &s) { return s.fluidCount <= kFluidWide && s.N <= 524288u ? kFluidLanes : 1u; }
+inline uint32_t fluidDeltaLanes(const Scene &s) { return s.fluidCount <= 32768u && s.N <= 524288u ? kFluidLanes : 1u; }
 inline unsigned fluidWideBlocks(size_t n, uint32_t lanes) { return fluidBlocksFor(n * lanes); }
 
 template <bool kExtras, uint32_t kLanes>
@@ -3645,7 +3646,7 @@ void launchFluidNeighborsDensity(const Scene &s, const Config &c, uint32_t iter,
     const Scene sp = withPositions(s, iter);
     float4 *Dk = (iter & 1u) ? s.Db : s.Da;
     const unsigned g = fluidBlocksFor(s.N);
-    const bool rebuild = s.P0 && iter > 0 && iter + kFluidRebuildAhead < s.fluidIterations;
+    const bool rebuild = s.P0 && iter > 0 && iter + fluidRebuildAhead(s.fluidCount) < s.fluidIterations;
     const uint32_t lanes = fluidLanes(s);
     if (s.sup && !walkCells && lanes > 1u) {
         if (s.fluidExtras) launchFluidWide<true, kFluidLanes>(sp, c, iter, Dk, rebuild, st);
@@ -3680,7 +3681,7 @@ void launchFluidDeltaApplyClamp(const Scene &s, uint32_t iter, float dt, const C
     const float4 *Dcur = (iter & 1u) ? s.Db : s.Da;
     float4 *Dnext = (iter & 1u) ? s.Da : s.Db;
     float4 *Pnext = s.Pb ? ((iter & 1u) ? s.P : s.Pb) : nullptr;
-    const uint32_t lanes = fluidLanes(s);
+    const uint32_t lanes = fluidDeltaLanes(s);
     if (lanes > 1u) {
         const Scene sp = withPositions(s, iter);
         const unsigned g = fluidWideBlocks(s.N, lanes);

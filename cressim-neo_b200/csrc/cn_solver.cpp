@@ -381,7 +381,7 @@ void layout(cn_solver *sv, cn::Arena &a, const cn_world_soa &w, const cn::Incide
         s.sup = a.take<uint32_t>(size_t(N) * s.supCap);
         s.supCount = a.take<uint32_t>(N);
         if (!sv->fluidXMoves) s.Pb = a.take<float4>(N);
-        if (sv->fluidXMoves || sv->fluidIt > 1u + cn::kFluidRebuildAhead) s.P0 = a.take<float4>(N);
+        if (sv->fluidXMoves || sv->fluidIt > 1u + cn::fluidRebuildAhead(s.fluidCount)) s.P0 = a.take<float4>(N);
         s.maxNbr = sv->desc.max_fluid_neighborhood;
         s.nbr = a.take<uint32_t>(std::max<size_t>(size_t(N) * s.maxNbr, 1));
         s.nbrCount = a.take<uint32_t>(N);

@@ -1,4 +1,4 @@
-"""Fluid kernels with eight lanes per particle and with one, on both sides of the size where the one takes over:
+"""Fluid kernels with eight lanes per particle and with one, on both sides of the sizes where the one takes over:
 each evaluates the oracle's expressions in its order, so states are equal bit for bit."""
 import numpy as np
 import pytest
@@ -9,9 +9,10 @@ from cn_physics import Solver, World, scenes, solver_desc
 pytestmark = pytest.mark.gpu
 
 
-# 22,528 fluid particles: eight lanes; 22,568: one; 1,000 beside 27,000 of tissue: eight, most slots of other kinds
+# 22,528 fluid particles: eight lanes; 22,568 and 32,768: one for the neighbours; 32,800: one; 1,000 beside 27,000 of
+# tissue: eight, most slots of other kinds
 @pytest.mark.parametrize("extras", [{}, dict(cohesion=0.02, surface_tension=0.5, vorticity=0.3)])
-@pytest.mark.parametrize("dims, tissue", [((22, 32, 32), 0), ((31, 28, 26), 0), ((10, 10, 10), 30)])
+@pytest.mark.parametrize("dims, tissue", [((22, 32, 32), 0), ((31, 28, 26), 0), ((32, 32, 32), 0), ((25, 32, 41), 0), ((10, 10, 10), 30)])
 def test_lanes_equal_the_oracle(dims, tissue, extras):
     w = World()
     sp = 0.05
