@@ -958,7 +958,8 @@ static void buildSolverTiles(cn_solver *sv, const cn_world_soa &w, const cn::Inc
     using In = cn::TileInput<decltype(edgeOf), decltype(tetOf), decltype(bendOf)>;
     const In in{N, w.positions_inv_mass, cls, edgeI, tetI, bendI, edgeOf, tetOf, bendOf};
     sv->tileContacts = contacts;
-    const uint32_t target = cn::tileTarget(tiled);
+    const bool fluid = size_t(std::count(w.kinds, w.kinds + N, uint32_t(CN_PARTICLE_FLUID))) > cn::kFluidWide;
+    const uint32_t target = cn::tileTarget(tiled, fluid);
     if (!target) return;
     try {
         sv->tileBuild = cn::buildTiles(in, target, cn::kTileSmemCap);

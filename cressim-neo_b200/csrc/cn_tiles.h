@@ -35,20 +35,23 @@ constexpr uint32_t kTileSmemCap = 112u << 10; // two tiles' CTAs on an SM
 //  * Large scenes fill whole waves of two CTAs an SM with tiles of at most 192 (a larger tile solves
 //    fewer constraints twice, but 340 leaves too few CTAs: 100K particles, 4 x 20 iterations, 2.4 ms at
 //    170, 2.9 at 96, 2.7 at 340, 4.0 with the per-family kernels).  16K of tissue and cloth, 2 x 20 iterations:
-//    1,217 us with the per-family kernels, 1,140 with tiles of 55, 1,206 of 64, 1,403 of 16; beside 130K of
-//    fluid 5,320 and 5,230.  Sized for all 146K particles of that world its tiles would be of 165: 4,250
-//    us against 4,130 (2 fluid iterations).
+//    1,217 us with the per-family kernels, 1,140 with tiles of 55, 1,206 of 64, 1,403 of 16.
+//  * Beside a fluid that fills the chip (`fluid`) work done twice is the fluid's time: no tiles from 1,536 to
+//    24,576 particles, of at least 144 above.  7K of tissue and cloth beside 50K of fluid, 2 x 20 iterations:
+//    3,555 us with the per-family kernels, 4,000 with tiles of 32, 3,610 of 96, 3,555 of 144; 17K beside 64K, 2 x 8:
+//    2,170, of 59 2,285, of 144 2,210; 38K beside 157K, 1 x 20: 2,600, of 129 2,585, of 144 2,580; 60K beside 130K,
+//    2 x 10: 7,754, of 144 7,690; 1K beside 130K, 2 x 20 (2 of the fluid): 2,267, of 16 2,130.
 //  * In between the per-family kernels stay, though the tiles measured faster there as well (4,096
 //    particles: 505 against 647 us): the frame graph of the 16^3 cube is held to one launch per
 //    phase by the schedule test, which the stages' two launches an iteration do not meet.
-inline uint32_t tileTarget(uint32_t n)
+inline uint32_t tileTarget(uint32_t n, bool fluid)
 {
-    if (n <= 3072u) return 16u;
-    if (n < 6144u) return 0u;
+    if (n <= (fluid ? 1536u : 3072u)) return 16u;
+    if (n < (fluid ? 24576u : 6144u)) return 0u;
     constexpr uint32_t kWave = 2u * 148u;
     uint32_t waves = 1u;
     while (n > kWave * waves * 192u) ++waves;
-    return std::max((n + kWave * waves - 1u) / (kWave * waves), 32u);
+    return std::max((n + kWave * waves - 1u) / (kWave * waves), fluid ? 144u : 32u);
 }
 
 // A vector whose new elements are left as they are: the lists are written, not zeroed first.
