@@ -221,3 +221,23 @@ def test_resident_colours_with_a_particle_named_twice(schedule):
     desc = solver_desc(substeps=2, default_iterations=3, enable_blocking_readback=0)
     desc.soft.xpbd_schedule = schedule
     _equal(*_states(w, desc))
+
+
+def test_rigid_candidates_in_one_block_and_in_launches():
+    # 512 particles take one block against any colliders, 720 against up to sixteen; launches are two more
+    count = {}
+    for n in ((8, 8, 8), (9, 8, 10)):
+        for colliders in (15, 40):
+            w = _block(n, pinned=False)
+            rng = np.random.default_rng(6)
+            for k in range(colliders):
+                b = w.add_rigid_body("static", position=tuple(float(c) for c in rng.uniform(-0.4, 0.4, 3)))
+                w.add_collider(b, ("sphere", "box")[k % 2], ((0.05,), (0.05, 0.05, 0.05))[k % 2])
+            desc = solver_desc(substeps=1, default_iterations=3, enable_blocking_readback=0, particle_rigid_pairs_per_particle=32)
+            gpu, ora = Solver(desc), cn_oracle.Oracle(desc, w.soa())
+            gpu.sync_world(w)
+            gpu.step(1.0 / 60.0)
+            ora.step(1.0 / 60.0)
+            _equal(gpu.read_particles(), ora.read_particles())
+            count[n[0], colliders] = gpu.graph_stats()[0]
+    assert count[9, 15] == count[8, 15] and count[9, 40] == count[8, 40] + 2
