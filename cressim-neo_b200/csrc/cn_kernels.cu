@@ -86,10 +86,6 @@ constexpr int kSoftBatchThreads = 128;
 inline unsigned softThreads(const Scene &s) { return s.wP.tiles ? kSoftBatchThreads : kSoftThreads; }
 inline unsigned softBlocksFor(size_t n) { return n == 0 ? 1u : unsigned((n + kSoftThreads - 1) / kSoftThreads); }
 inline unsigned softGridFor(const WorkList &w, size_t n) { return w.tiles ? w.grid : softBlocksFor(n); }
-inline unsigned softApplyGrid(const Scene &s, uint2 win)
-{
-    return s.wP.tiles ? gridFor(s.wP, s.N) : softBlocksFor(win.y > win.x ? size_t(win.y - win.x) * 4u : 0u);
-}
 
 // forEachElem for loops that one block runs over a small family (rigid bodies, colliders).
 template <class F> __device__ __forceinline__ void forEachInBlock(const WorkList &w, uint32_t n, F &&f)
@@ -2017,11 +2013,18 @@ struct GatherLane {
 // physics_soft_apply_bend_corrections.cs.hlsl:9-51, physics_strand_apply_distance_corrections.cs.hlsl:9-38.
 // A single world applies over `win`, the particles [lo, hi) that the family touches (bodies are
 // contiguous in the particle order; the others have no records and keep x); a batch over its tiles.
-__global__ void __launch_bounds__(kThreads) k_applyGather(Scene s, const uint2 *ranges, const float4 *corr, uint2 win)
+// `wide`: a single world's four lanes per particle (gatherWide).  One kernel for the three: alone the
+// four lanes are compiled for 32 registers, without their sixteen records in flight (16^3 cube 253 -> 263 us).
+__global__ void __launch_bounds__(kThreads) k_applyGather(Scene s, const uint2 *ranges, const float4 *corr, uint2 win, bool wide)
 {
-    if (s.wP.tiles) {
+    if (!wide) {
         pdlEnter();
-        forEachElem(s.wP, s.N, [&](uint32_t i) { applyGatherAt(s, ranges, corr, i); });
+        if (s.wP.tiles) {
+            forEachElem(s.wP, s.N, [&](uint32_t i) { applyGatherAt(s, ranges, corr, i); });
+            return;
+        }
+        const uint32_t i = win.x + blockIdx.x * blockDim.x + threadIdx.x;
+        if (i < win.y) applyGatherAt(s, ranges, corr, i);
         return;
     }
     const GatherLane g(s, ranges, win.x + (blockIdx.x * blockDim.x + threadIdx.x) / kGatherLanes, win.y);
@@ -2941,9 +2944,9 @@ __global__ void __launch_bounds__(kThreads) k_rigidContacts(Scene s, Config cfg,
 // position, its candidate pairs and the colliders, so running them in the same thread right after
 // its gather (over the same particles as the two per-phase kernels: the tet window, then every
 // particle) gives their results bit for bit with one launch and one pass over x fewer.
-__global__ void __launch_bounds__(kThreads) k_applyTetsRigidContacts(Scene s, Config cfg)
+__global__ void __launch_bounds__(kThreads) k_applyTetsRigidContacts(Scene s, Config cfg, bool wide)
 {
-    if (!s.wP.tiles) { // a single world: the four-lane gather, its first lane runs the contacts
+    if (wide) { // the four-lane gather, its first lane runs the contacts
         const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / kGatherLanes;
         GatherLane g(s, s.tetRanges, i, s.N);
         ContactRange range{};
@@ -2963,7 +2966,7 @@ __global__ void __launch_bounds__(kThreads) k_applyTetsRigidContacts(Scene s, Co
     // the gathered position goes to the contacts in registers: x is read and written once
     forEachElem(s.wP, s.N, [&](uint32_t i) {
         float4 p = s.x[i];
-        p = gatheredPosition(s.tetRanges, s.tetCorr, i, p);
+        if (s.wP.tiles || (i >= s.tetWin.x && i < s.tetWin.y)) p = gatheredPosition(s.tetRanges, s.tetCorr, i, p);
         rigidContactsFrom(s, cfg, true, i, p, contactRange(s, i));
     });
 }
@@ -4620,6 +4623,20 @@ bool launchSoftIteration(const Scene &s, float dt, const Config &c, cudaStream_t
     return launchSoftFamilies(s, dt, c, st, kAllFamilies, first, rigidContacts);
 }
 
+// Four lanes per particle of a gather over n particles of a single world: up to 32,768, from where on the
+// chip has threads enough with one each.  Frames of 2 substeps x 10 iterations, one lane against four: tissue of
+// 4,096 311 -> 263 us, of 27,000 (beside cloth, by family) 985 -> 940, of 46,656 1,140 -> 1,145, of 97,336 1,702 -> 1,829;
+// strands of 8,256 particles 675 -> 633, of 25,800 728 -> 730, of 38,700 766 -> 786, of 129,000 1,066 -> 1,220.
+inline bool gatherWide(const Scene &s, size_t n) { return !s.wP.tiles && n <= 32768u; }
+
+static void launchGather(const Scene &s, const uint2 *ranges, const float4 *corr, uint2 win, cudaStream_t st)
+{
+    const size_t n = win.y > win.x ? win.y - win.x : 0u;
+    const bool wide = gatherWide(s, n);
+    const unsigned grid = s.wP.tiles ? gridFor(s.wP, s.N) : softBlocksFor(n * (wide ? kGatherLanes : 1u));
+    launchPdl(k_applyGather, grid, softThreads(s), st, s, ranges, corr, win, wide);
+}
+
 bool launchSoftFamilies(const Scene &s, float dt, const Config &c, cudaStream_t st, uint32_t families, bool first,
                         bool rigidContacts)
 {
@@ -4627,7 +4644,7 @@ bool launchSoftFamilies(const Scene &s, float dt, const Config &c, cudaStream_t 
     auto on = [&](uint32_t f) { return ((families >> f) & 1u) != 0u; };
     if (s.E && on(kFamEdges)) {
         launchPdl(k_solveEdges, softGridFor(s.wE, s.E), softThreads(s), st, s, dt, relax, first);
-        launchPdl(k_applyGather, softApplyGrid(s, s.edgeWin), softThreads(s), st, s, s.edgeRanges, s.edgeCorr, s.edgeWin);
+        launchGather(s, s.edgeRanges, s.edgeCorr, s.edgeWin, st);
     }
     if (s.S && on(kFamSegments)) {
         launchPdl(k_solveSegments, softBlocksFor(s.S), softThreads(s), st, s, dt, relax);
@@ -4636,7 +4653,7 @@ bool launchSoftFamilies(const Scene &s, float dt, const Config &c, cudaStream_t 
     if ((s.Bn || s.D) && on(kFamBends)) {
         if (s.Bn) launchPdl(k_solveBends, softBlocksFor(s.Bn), softThreads(s), st, s, dt, relax);
         if (s.D) launchPdl(k_solveDihedrals, softBlocksFor(s.D), softThreads(s), st, s, dt, relax);
-        launchPdl(k_applyGather, softApplyGrid(s, s.bendWin), softThreads(s), st, s, s.bendRanges, s.bendCorr, s.bendWin);
+        launchGather(s, s.bendRanges, s.bendCorr, s.bendWin, st);
     }
     if (s.J && on(kFamJoints)) {
         launchPdl(k_solveJoints, softBlocksFor(s.J), softThreads(s), st, s, dt, relax);
@@ -4644,15 +4661,16 @@ bool launchSoftFamilies(const Scene &s, float dt, const Config &c, cudaStream_t 
     }
     if (s.SD && on(kFamDistances)) {
         launchPdl(k_solveDistances, softBlocksFor(s.SD), softThreads(s), st, s, dt, relax);
-        launchPdl(k_applyGather, softApplyGrid(s, s.segWin), softThreads(s), st, s, s.segRanges, s.distCorr, s.segWin);
+        launchGather(s, s.segRanges, s.distCorr, s.segWin, st);
     }
     if (s.T && on(kFamTets)) {
         launchPdl(k_solveTets, softGridFor(s.wT, s.T), softThreads(s), st, s, dt, relax, first);
         if (rigidContacts && s.N) {
-            launchPdl(k_applyTetsRigidContacts, softGridFor(s.wP, size_t(s.N) * kGatherLanes), softThreads(s), st, s, c);
+            const bool wide = gatherWide(s, s.N);
+            launchPdl(k_applyTetsRigidContacts, softGridFor(s.wP, size_t(s.N) * (wide ? kGatherLanes : 1u)), softThreads(s), st, s, c, wide);
             return true;
         }
-        launchPdl(k_applyGather, softApplyGrid(s, s.tetWin), softThreads(s), st, s, s.tetRanges, s.tetCorr, s.tetWin);
+        launchGather(s, s.tetRanges, s.tetCorr, s.tetWin, st);
     }
     return false;
 }

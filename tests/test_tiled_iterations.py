@@ -128,6 +128,19 @@ def test_disabled_edges_and_a_hub():
     assert _launches(w, desc) == 2
 
 
+# a particle with more edges than a tile's records hold: the families' own kernels, gathers of four lanes per particle up
+# to 32,768 particles and of one above
+@pytest.mark.parametrize("n", [(31, 33, 32), (32, 33, 32)])
+def test_families_beside_a_hub_over_the_tiles_limit(n):
+    w = _block(n)
+    e = w.array("edges")
+    e[:1100, 0] = 5000
+    e[:, 1][e[:, 0] == e[:, 1]] = 5001
+    desc = solver_desc(substeps=1, default_iterations=3, enable_blocking_readback=0, soft_internal_relaxation=0.001)
+    _equal(*_states(w, desc))
+    assert _launches(w, desc) == 4
+
+
 def test_edges_alone():
     rng = np.random.default_rng(3)
     w = World()
