@@ -997,7 +997,7 @@ __device__ __forceinline__ bool supersetsDue(const Scene &s, uint32_t iter)
 // Whether they are built anew.  An iteration whose lists did not last through the next one (noteSuperset)
 // leaves it, in the substeps that follow, until the move since the last iteration is below the bound: a
 // fluid that outruns its lists every time only pays for recording them (4 iterations, late frames of a
-// 262K-particle gas 2,400 us a frame without, 2,530 with, a pressed block of 110K 5,050 and 5,560).
+// pressed block of 110K particles 5,050 us a frame without, 5,560 with).
 __device__ __forceinline__ bool supersetsAnew(const Scene &s, uint32_t iter)
 {
     if (!supersetsDue(s, iter)) return false;
