@@ -4682,8 +4682,9 @@ namespace {
 
 // One CTA per tile, two on an SM (the contacts' registers; 3 or 4 a SM spill and measured 4-14 % slower).
 // What bounds a stage: a small scene, the chain wait -> positions -> solve (some 250 dependent
-// instructions for a tet) -> sum -> store; a large one, the same chain over too few warps (ncu, 100K
-// particles: issue 43 %, long scoreboard 7.4 per issue, DRAM 13-20 % of peak).  Against the four per-family
+// instructions for a tet) -> sum -> store; a large one, the same chain over too few warps (ncu, 97K
+// particles: issue 51 % in the edges' stage and 35 % in the tets' with contacts, long scoreboard 4.6 and 3.9 per
+// issue, DRAM 11-13 % of peak).  Against the four per-family
 // launches an iteration it saves the correction records' trips through L2 (128 B a tet, 64 B an edge,
 // scattered) and two launches: 100K particles 3.97 -> 2.29 ms a frame of 80 iterations, a cloth of 12.5K
 // 1.32 -> 0.75 ms, 216 particles in contact 1.24 -> 0.66 ms.
