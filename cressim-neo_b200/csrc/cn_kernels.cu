@@ -1221,6 +1221,7 @@ __global__ void __launch_bounds__(kFluidThreads, (kExtras ? 4 : 5) * (256 / kFlu
 // 512K particles at rest: 8,530 us a frame so, 8,940 with one walk for both lists, 9,000 inlined).
 template <bool kExtras> __device__ __noinline__ void recordSuperset(const Scene &s, const Config &cfg, uint32_t slot)
 {
+    if ((s.sInfo[slot] & kFluidBit) == 0u) return;
     // a warp with an overflowed list among its own would filter and walk: it walks until the next substep
     if (__any_sync(__activemask(), s.supCount[slot] > s.supCap)) {
         s.supCount[slot] = s.supCap + 1u;
